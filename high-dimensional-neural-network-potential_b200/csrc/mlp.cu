@@ -74,186 +74,174 @@ __global__ void __launch_bounds__(kThreads) k_mlp(Batch b, DevModel m, int maxw)
 
 // ---------------------------------------------------------------- FP64 tensor cores
 // The FP64 networks on the FP64 tensor cores: mma.sync m8n8k4 f64 (tcgen05
-// has no FP64 kind), a warp per 8 atoms of one element.  The first layer's
-// GEMM (8 x nin) x (nin x 32) and the input gradient dE/dG = delta_1 W_1,
-// (8 x 32) x (32 x nin), carry ~90 % of the multiply-adds; the hidden and
-// output layers (widths <= 32) run on the lanes from shared memory.  Same
-// formulas as mlp_tile (neuralNetworks.f90:94-158); the sums of the two
-// GEMMs run in the tensor cores' order.
+// has no FP64 kind), tiles of 8 atoms of one element.  Layer 1 is the GEMM
+// (8 x nin) x (nin x 32), dE/dG = delta_1 W_1 the GEMM (8 x 32) x (32 x nin).
+// Same formulas as mlp_tile (neuralNetworks.f90:94-158).
 //   fragments (thread t): A[t/4][t%4], B[k = t%4][n = t/4],
 //   C[t/4][2 (t%4) + v], v = 0, 1
+// Two kernels share the work by batch size (launch_mlp):
+//   k_mlp_split     a block of 8 warps per tile: the warps split layer 1's
+//                   inputs and the columns of dE/dG, so that one tile's chain
+//                   of loads is short.
+//   k_mlp_resident  a block per SM keeps the weights of one element in shared
+//                   memory and its warps take a tile each.
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double bb) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
                  : "+d"(c[0]), "+d"(c[1])
                  : "d"(a), "d"(bb));
 }
 
-constexpr int kDW = 4;   // warps per block
-constexpr int kDH = 32;  // widest layer the kernel takes
-constexpr int kDR = 8;   // atoms per warp
+constexpr int kDW = 8;   // warps per block of k_mlp_split, one per atom of the tile
+constexpr int kRW = 10;  // warps per block of k_mlp_resident
+constexpr int kDH = 32;  // widest layer the kernels take
+constexpr int kDR = 8;   // atoms per tile
+// row stride of the activation rows: four rows of four doubles (the A
+// fragment's half-warp) fall on distinct banks
+constexpr int kDS = 36;
 
-// Row stride of the per-warp activation rows: the widest layer + 1, odd.
-__host__ __device__ inline int dmma_stride(int maxw) { return (maxw + 1) | 1; }
-// per warp: act'(c_l) of every layer and two rotating rows (activations in
-// the forward pass, deltas in the backward pass), [8][stride] each
-__host__ __device__ inline int dmma_warp_doubles(int L, int stride) { return (L + 2) * kDR * stride; }
+// tiles of 8 atoms of element x
+__device__ __forceinline__ int el_tiles(const Batch& b, int x) {
+    return (b.el_start[x + 1] - b.el_start[x] + kDR - 1) / kDR;
+}
 
-__global__ void __launch_bounds__(32 * kDW, 6) k_mlp_dmma(Batch b, DevModel m, int S) {
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// shared memory of k_mlp_split in doubles: hidden weights with odd row
+// strides, activations/deltas [2][8][kDS], act'(c_l) [L][8][kDS], layer-1
+// partial sums [8 warps][8][kDS]
+__host__ __device__ inline int split_hidden_doubles(const DevModel& m) {
+    int n = 0;
+    for (int l = 1; l < m.nlayers; ++l) n += m.width[l] * (m.width[l + 1] | 1);
+    return (n + 1) & ~1;  // what follows starts on a 16-byte boundary
+}
+__host__ __device__ inline int split_doubles(const DevModel& m) {
+    return split_hidden_doubles(m) + (2 + m.nlayers + kDW) * kDR * kDS;
+}
+
+// Bound by the latency of one tile's chain: element and atom lookup, G and
+// W1 loads, the layers, dE/dG.  The 8 warps take 1/8 of layer 1's k-steps
+// each (partial sums added in warp order) and every 8th pair of dE/dG
+// columns; a thread owns one (atom, neuron) of the hidden layers, whose
+// weights arrive in shared memory while layer 1 multiplies.  Cold, a warp
+// per tile with all of it in one chain took 113 us for the 768-atom cell
+// (96 tiles).
+__global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
     extern __shared__ __align__(16) double dsm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
     const int L = m.nlayers;
-    // locate (element, tile of 8 atoms) of this warp
-    int tile = blockIdx.x * kDW + wib, e = -1, t0 = 0, cnt = 0;
+    int tile = blockIdx.x, e = -1, t0 = 0, cnt = 0;
     for (int x = 0; x < m.nel; ++x) {
-        const int n = b.el_start[x + 1] - b.el_start[x];
-        const int nt = (n + kDR - 1) / kDR;
+        const int nt = el_tiles(b, x);
         if (tile < nt) {
             e = x;
             t0 = b.el_start[x] + tile * kDR;
-            cnt = min(kDR, n - tile * kDR);
+            cnt = min(kDR, b.el_start[x + 1] - t0);
             break;
         }
         tile -= nt;
     }
-    if (e < 0) return;  // uniform per warp
-    double* ws = dsm + (size_t)wib * dmma_warp_doubles(L, S);
-    auto da = [&](int l) { return ws + l * kDR * S; };          // act'(c_l)
-    auto yb = [&](int p) { return ws + (L + p) * kDR * S; };    // rotating rows
+    if (e < 0) return;  // uniform per block
+    double* hw = dsm;
+    double* yb = hw + split_hidden_doubles(m);  // two rotating row sets
+    double* da = yb + 2 * kDR * kDS;
+    double* part = da + L * kDR * kDS;
+    {
+        double* dst = hw;
+        for (int l = 1; l < L; ++l) {
+            const int win = m.width[l], wout = m.width[l + 1], st = wout | 1;
+            const double* WT = m.wt + m.w_off[e * L + l];  // [win][wout]
+            for (int idx = tid; idx < win * wout; idx += 32 * kDW) cp_async8(dst + (idx / wout) * st + idx % wout, WT + idx);
+            dst += win * st;
+        }
+    }
     const int r = lane >> 2, q = lane & 3;
     const int atom = r < cnt ? b.el_atoms[t0 + r] : -1;
     const int nin = m.nin_el[e], nsf = m.nsf_max, H1 = m.width[1];
-    // layer 1: C[8 x 32] = G[8 x nin] W1^T on the tensor cores; the next
-    // k-step's operands are loaded while this one multiplies
-    double acc[4][2];
+    {
+        double acc[4][2];
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
-    const double* grow = atom >= 0 ? b.G + (size_t)atom * nsf : nullptr;
-    const double* F = m.dm_fwd + m.dm_off_f[e] + lane;  // [ks][nt][32]
-    const int KS = (nin + 3) >> 2;
-    // operands of k-step ks (zero A and no B load beyond the last step)
-    auto load = [&](int ks, double& a, double (&bf)[4]) {
-        const int k = 4 * ks + q;
-        a = (grow && k < nin) ? __ldg(grow + k) : 0.0;
-        if (ks < KS) {
+        for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+        const double* grow = atom >= 0 ? b.G + (size_t)atom * nsf : nullptr;
+        const double* F = m.dm_fwd + m.dm_off_f[e] + lane;  // [ks][nt][32]
+        const int KS = (nin + 3) >> 2, per = (KS + kDW - 1) / kDW;
+        const int k0 = wib * per, k1 = min(KS, k0 + per);
+#pragma unroll 5
+        for (int ks = k0; ks < k1; ++ks) {
+            const int k = 4 * ks + q;
+            const double a = (grow && k < nin) ? __ldg(grow + k) : 0.0;
             const double* f = F + (size_t)ks * 128;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) bf[nt] = __ldg(f + nt * 32);
+            for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], a, __ldg(f + nt * 32));
         }
-    };
-    // two k-steps in flight: the operands of ks + 2 are loaded while ks
-    // multiplies (two register sets, the loop unrolled by two)
-    double a0 = 0.0, a1 = 0.0, b0[4] = {0.0, 0.0, 0.0, 0.0}, b1[4] = {0.0, 0.0, 0.0, 0.0};
-    load(0, a0, b0);
-    load(1, a1, b1);
-    for (int ks = 0; ks < KS; ks += 2) {
-        {
-            const double a = a0;
-            double bb[4];
+        double* pw = part + wib * kDR * kDS + r * kDS + 2 * q;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) bb[nt] = b0[nt];
-            if (ks + 2 < KS) load(ks + 2, a0, b0);
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], a, bb[nt]);
-        }
-        if (ks + 1 < KS) {
-            const double a = a1;
-            double bb[4];
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) bb[nt] = b1[nt];
-            if (ks + 3 < KS) load(ks + 3, a1, b1);
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], a, bb[nt]);
-        }
+        for (int nt = 0; nt < 4; ++nt) *reinterpret_cast<double2*>(pw + 8 * nt) = make_double2(acc[nt][0], acc[nt][1]);
     }
-    {
-        const double* b1 = m.b + m.b_off[e * L];
+    cp_async_wait();
+    __syncthreads();
+    // thread = (atom wib, neuron lane) from here to the deltas
+    const int row = wib * kDS + lane;
+    if (lane < H1) {
+        double c = part[row];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int v = 0; v < 2; ++v) {
-                const int col = nt * 8 + 2 * q + v;
-                if (col < H1) {
-                    const double cv = acc[nt][v] + b1[col];
-                    const double yv = act_f(m.act[0], cv);
-                    yb(0)[r * S + col] = yv;
-                    da(0)[r * S + col] = act_d(m.act[0], cv, yv);
-                }
-            }
+        for (int w = 1; w < kDW; ++w) c += part[w * kDR * kDS + row];
+        c += m.b[m.b_off[e * L] + lane];
+        const double y = act_f(m.act[0], c);
+        yb[row] = y;
+        da[row] = act_d(m.act[0], c, y);
     }
     __syncwarp();
-    // hidden and output layers: lane = output neuron, the warp's 8 atoms
+    const double* W = hw;
     for (int l = 1; l < L; ++l) {
-        const int win = m.width[l], wout = m.width[l + 1];
-        // transposed weights [win][wout]: the lanes' loads of one input are
-        // one coalesced row
-        const double* WT = m.wt + m.w_off[e * L + l];
-        const double* bl = m.b + m.b_off[e * L + l];
-        const double* yin = yb((l - 1) & 1);
-        double* yout = yb(l & 1);
+        const int win = m.width[l], wout = m.width[l + 1], st = wout | 1;
+        const double* yin = yb + ((l - 1) & 1) * kDR * kDS + wib * kDS;
         if (lane < wout) {
-            double sacc[kDR];
-#pragma unroll
-            for (int rr = 0; rr < kDR; ++rr) sacc[rr] = 0.0;
-            // unrolled so that several weight loads are in flight (they come
-            // from L2: the shared memory of 6 blocks leaves no L1)
+            double c = 0.0;
 #pragma unroll 5
-            for (int i = 0; i < win; ++i) {
-                const double w = __ldg(WT + (size_t)i * wout + lane);
-#pragma unroll
-                for (int rr = 0; rr < kDR; ++rr) sacc[rr] += w * yin[rr * S + i];
-            }
-#pragma unroll
-            for (int rr = 0; rr < kDR; ++rr) {
-                const double cv = sacc[rr] + bl[lane];
-                const double yv = act_f(m.act[l], cv);
-                yout[rr * S + lane] = yv;
-                da(l)[rr * S + lane] = act_d(m.act[l], cv, yv);
-            }
+            for (int i = 0; i < win; ++i) c += W[i * st + lane] * yin[i];
+            c += m.b[m.b_off[e * L + l] + lane];
+            const double y = act_f(m.act[l], c);
+            yb[(l & 1) * kDR * kDS + row] = y;
+            da[l * kDR * kDS + row] = act_d(m.act[l], c, y);
         }
+        W += win * st;
         __syncwarp();
     }
-    // atomic energies, then the rotating rows carry the deltas
-    if (lane < cnt) b.atE[b.el_atoms[t0 + lane]] = yb((L - 1) & 1)[lane * S] + m.atom_energy[e];
+    if (lane == 0 && wib < cnt)
+        b.atE[b.el_atoms[t0 + wib]] = yb[((L - 1) & 1) * kDR * kDS + row] + m.atom_energy[e];
     __syncwarp();
-    double* dcur = yb(0);
-    double* dnext = yb(1);
-    {
-        const int w = m.width[L];  // gradOut = 1
-        if (lane < w)
-#pragma unroll
-            for (int rr = 0; rr < kDR; ++rr) dcur[rr * S + lane] = da(L - 1)[rr * S + lane];
-    }
+    // deltas in the rotating rows (gradOut = 1)
+    double* dcur = yb;
+    double* dnext = yb + kDR * kDS;
+    const double* dl = da + (L - 1) * kDR * kDS + row;  // act'(c_l) of this thread's neuron
+    if (lane < m.width[L]) dcur[row] = *dl;
     __syncwarp();
     for (int l = L - 1; l >= 1; --l) {
-        const int wout = m.width[l + 1], wi = m.width[l];
-        const double* W = m.w + m.w_off[e * L + l];  // [wout][wi]
-        if (lane < wi) {
-            // each weight loaded once for the warp's 8 atoms (same sum order)
-            double sv[kDR];
-#pragma unroll
-            for (int rr = 0; rr < kDR; ++rr) sv[rr] = 0.0;
+        const int win = m.width[l], wout = m.width[l + 1], st = wout | 1;
+        W -= win * st;
+        dl -= kDR * kDS;
+        if (lane < win) {
+            double s = 0.0;
 #pragma unroll 5
-            for (int o = 0; o < wout; ++o) {
-                const double w = __ldg(W + (size_t)o * wi + lane);
-#pragma unroll
-                for (int rr = 0; rr < kDR; ++rr) sv[rr] += dcur[rr * S + o] * w;
-            }
-#pragma unroll
-            for (int rr = 0; rr < kDR; ++rr) dnext[rr * S + lane] = sv[rr] * da(l - 1)[rr * S + lane];
+            for (int o = 0; o < wout; ++o) s += dcur[wib * kDS + o] * W[lane * st + o];
+            dnext[row] = s * *dl;
         }
         __syncwarp();
         double* t = dcur;
         dcur = dnext;
         dnext = t;
     }
-    // dE/dG = delta_1 W1: C[8 x nin] = A[8 x 32] B[32 x nin] on the tensor cores
+    __syncthreads();
     double afr[kDH / 4];
 #pragma unroll
-    for (int ks = 0; ks < kDH / 4; ++ks) afr[ks] = (4 * ks + q < H1) ? dcur[r * S + 4 * ks + q] : 0.0;
-    // two n-tiles per iteration (independent accumulator chains)
+    for (int ks = 0; ks < kDH / 4; ++ks) afr[ks] = (4 * ks + q < H1) ? dcur[r * kDS + 4 * ks + q] : 0.0;
     const double* Bw = m.dm_bwd + m.dm_off_b[e] + lane;  // [nb][ks][32]
     const int KB = (H1 + 3) >> 2, NB = (nin + 7) >> 3;
-    for (int nb = 0; nb < NB; nb += 2) {
+    for (int nb = 2 * wib; nb < NB; nb += 2 * kDW) {
         const bool two = nb + 1 < NB;  // uniform
         const double* b0 = Bw + (size_t)nb * KB * 32;
         const double* b1 = b0 + KB * 32;
@@ -272,6 +260,244 @@ __global__ void __launch_bounds__(32 * kDW, 6) k_mlp_dmma(Batch b, DevModel m, i
                 const int col = nb * 8 + 2 * q + v;
                 if (col < nin) drow[col] = c0[v];
                 if (two && col + 8 < nin) drow[col + 8] = c1[v];
+            }
+        }
+    }
+}
+
+// Shared memory of k_mlp_resident in doubles: W1 in the fragment orders of
+// layer 1 and of dE/dG, the later layers' weights in those of their forward
+// and backward products, biases, and per warp one activation/delta row set
+// and act'(c_l) of the layers but the last.
+struct DmmaLayout {
+    int f1, b1, hid, bias, warps, total;
+};
+__host__ __device__ inline DmmaLayout dmma_layout(const DevModel& m, int nin) {
+    DmmaLayout o;
+    const int H1 = m.width[1], L = m.nlayers;
+    o.f1 = 0;
+    o.b1 = o.f1 + ((nin + 7) >> 3) * 8 * 32;
+    o.hid = o.b1 + ((nin + 7) >> 3) * ((H1 + 3) >> 2) * 32;
+    int h = 0;
+    for (int l = 1; l < L; ++l) {
+        const int wi = m.width[l], wo = m.width[l + 1];
+        h += (((wi + 3) >> 2) * ((wo + 7) >> 3) + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
+    }
+    o.bias = o.hid + h;
+    o.warps = o.bias + L * kDH;
+    o.total = o.warps + kRW * L * kDR * kDS;
+    return o;
+}
+
+// C[8 x 8 NT] += A[8 x 4 KS] B with the A fragments read from the rows at
+// `rows` and the B fragments [ks][nt][32] at `B`, both in shared memory;
+// columns of A beyond `k` read as zero.
+__device__ __forceinline__ void rows_gemm(double (&acc)[4][2], const double* rows, int k, const double* B, int NT, int r,
+                                          int q, int lane) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+    const int KS = (k + 3) >> 2;
+#pragma unroll 2
+    for (int ks = 0; ks < KS; ++ks) {
+        const double a = 4 * ks + q < k ? rows[r * kDS + 4 * ks + q] : 0.0;
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+            if (nt < NT) dmma(acc[nt], a, B[(ks * NT + nt) * 32 + lane]);
+    }
+}
+
+// Bound by the FP64 tensor cores (about 590 m8n8k4 per tile of a
+// 280-25-25-1 network; 0.7 ms for the 758,676 atoms of the 4096-structure
+// batch at the FP64 GEMM rate) and by G in, dE/dG out (0.5 ms of HBM).  Both
+// orders of W1 (134 KB) and the later layers stay in shared memory, a block
+// per SM over a contiguous share of the tiles, so every B fragment is a
+// conflict-free shared load; every layer is a tensor-core product.  A
+// fragments come straight from the G rows, 12 pairs of k-steps (two
+// consecutive inputs per 16-byte load) ahead, across tiles too.  With the
+// weights from L2 and a warp per tile this pass took 2.92 ms; this form takes
+// 1.95.
+// kVec: G and dE/dG rows start on 16-byte boundaries (nsf_max even).
+template <bool kVec>
+__global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel m, int nin_max) {
+    extern __shared__ __align__(16) double dsm[];
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+    const int L = m.nlayers, H1 = m.width[1], nsf = m.nsf_max;
+    const DmmaLayout lo = dmma_layout(m, nin_max);
+    double* yrow = dsm + lo.warps + wib * L * kDR * kDS;
+    double* da = yrow + kDR * kDS;
+    const int r = lane >> 2, q = lane & 3;
+    const int KB = (H1 + 3) >> 2;
+    long long T = 0;
+    for (int x = 0; x < m.nel; ++x) T += el_tiles(b, x);
+    const int first = (int)(T * blockIdx.x / gridDim.x), end = (int)(T * (blockIdx.x + 1) / gridDim.x);
+    constexpr int kCh = 12;  // pairs of k-steps in flight
+    int base = 0;
+    for (int e = 0; e < m.nel; ++e) {
+        const int nte = el_tiles(b, e);
+        const int s0 = max(first, base) - base, s1 = min(end, base + nte) - base;
+        base += nte;
+        if (s0 >= s1) continue;  // uniform per block
+        const int nin = m.nin_el[e], KP = (nin + 7) >> 3, NB = KP;
+        __syncthreads();  // the previous element's weights are no longer read
+        {
+            // [2 p + v][nt][t] = W1[8 nt + t/4][8 p + 2 (t%4) + v], from the
+            // packed k-steps of four consecutive inputs (coalesced reads; the
+            // steps beyond the last one of an odd count are zero)
+            const double* src = m.dm_fwd + m.dm_off_f[e];
+            const int nf1 = ((nin + 3) >> 2) * 128;
+            for (int idx = tid; idx < KP * 256; idx += 32 * kRW) {
+                const int t = idx & 31, nt = (idx >> 5) & 3, ks = idx >> 7;
+                const int kk = 4 * (ks & 1) + (t & 3);
+                double* dst = dsm + lo.f1 + ((((ks & ~1) | (kk & 1)) * 4 + nt) << 5) + ((t & ~3) | (kk >> 1));
+                if (idx < nf1) cp_async8(dst, src + idx);
+                else *dst = 0.0;
+            }
+            for (int idx = tid; idx < NB * KB * 32; idx += 32 * kRW)
+                cp_async8(dsm + lo.b1 + idx, m.dm_bwd + m.dm_off_b[e] + idx);
+            double* h = dsm + lo.hid;
+            for (int l = 1; l < L; ++l) {
+                const int wi = m.width[l], wo = m.width[l + 1];
+                const double* W = m.w + m.w_off[e * L + l];  // [wo][wi]
+                const int NT = (wo + 7) >> 3, nf = ((wi + 3) >> 2) * NT * 32;
+                for (int idx = tid; idx < nf; idx += 32 * kRW) {
+                    const int t = idx & 31, n = ((idx >> 5) % NT) * 8 + (t >> 2), k = 4 * ((idx >> 5) / NT) + (t & 3);
+                    h[idx] = (n < wo && k < wi) ? W[(size_t)n * wi + k] : 0.0;
+                }
+                h += nf;
+                const int NT2 = (wi + 7) >> 3, nb = ((wo + 3) >> 2) * NT2 * 32;
+                for (int idx = tid; idx < nb; idx += 32 * kRW) {
+                    const int t = idx & 31, n = ((idx >> 5) % NT2) * 8 + (t >> 2), k = 4 * ((idx >> 5) / NT2) + (t & 3);
+                    h[idx] = (k < wo && n < wi) ? W[(size_t)k * wi + n] : 0.0;
+                }
+                h += nb;
+            }
+            for (int idx = tid; idx < L * kDH; idx += 32 * kRW) {
+                const int l = idx / kDH, n = idx % kDH;
+                dsm[lo.bias + idx] = n < m.width[l + 1] ? m.b[m.b_off[e * L + l] + n] : 0.0;
+            }
+        }
+        cp_async_wait();
+        __syncthreads();
+        const double* F = dsm + lo.f1 + lane;
+        const double* Bw = dsm + lo.b1 + lane;
+        const int a0 = b.el_start[e], a1 = b.el_start[e + 1];
+        auto atom_of = [&](int tile) {
+            const int at = a0 + tile * kDR + r;
+            return (tile < s1 && at < a1) ? b.el_atoms[at] : -1;
+        };
+        // inputs 8 p + 2 q and the next of an atom's row, zero beyond nin
+        auto load = [&](int atom, int p, double2& v) {
+            v = make_double2(0.0, 0.0);
+            const int k = 8 * p + 2 * q;
+            if (atom >= 0 && p < KP && k < nin) {
+                const double* g = b.G + (size_t)atom * nsf + k;
+                if (kVec) v = __ldcs(reinterpret_cast<const double2*>(g));
+                else {
+                    v.x = __ldcs(g);
+                    if (k + 1 < nin) v.y = __ldcs(g + 1);
+                }
+                if (k + 1 >= nin) v.y = 0.0;
+            }
+        };
+        // the ring holds kCh pairs of k-steps ahead: a slot is loaded again as
+        // soon as it has been multiplied, at the end of a row with the next
+        // tile's first inputs
+        double2 an[kCh];
+        int atom_n = atom_of(s0 + wib);
+#pragma unroll
+        for (int i = 0; i < kCh; ++i) load(atom_n, i, an[i]);
+        for (int tile = s0 + wib; tile < s1; tile += kRW) {
+            const int atom = atom_n;
+            atom_n = atom_of(tile + kRW);
+            double acc[4][2];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+            for (int p0 = 0; p0 < KP; p0 += kCh) {
+                const bool more = p0 + kCh < KP;
+                const int an_atom = more ? atom : atom_n, an_p = more ? p0 + kCh : 0;
+#pragma unroll
+                for (int i = 0; i < kCh; ++i) {
+                    if (p0 + i < KP) {
+                        const double* f = F + (size_t)(p0 + i) * 256;
+#pragma unroll
+                        for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], an[i].x, f[nt * 32]);
+#pragma unroll
+                        for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], an[i].y, f[128 + nt * 32]);
+                    }
+                    load(an_atom, an_p + i, an[i]);
+                }
+            }
+            const double* h = dsm + lo.hid;
+            for (int l = 0; l < L; ++l) {
+                const int wo = m.width[l + 1], NT = (wo + 7) >> 3;
+                if (l > 0) {
+                    const int wi = m.width[l];
+                    rows_gemm(acc, yrow, wi, h, NT, r, q, lane);
+                    h += (((wi + 3) >> 2) * NT + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
+                    __syncwarp();
+                }
+                const char act = m.act[l];
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const int col = nt * 8 + 2 * q + v;
+                        if (col < wo) {
+                            const double c = acc[nt][v] + dsm[lo.bias + l * kDH + col];
+                            const double y = act_f(act, c);
+                            const double d = act_d(act, c, y);
+                            if (l + 1 < L) {
+                                yrow[r * kDS + col] = y;
+                                da[(l * kDR + r) * kDS + col] = d;
+                            } else {
+                                yrow[r * kDS + col] = d;  // gradOut = 1
+                                if (atom >= 0 && col == 0) b.atE[atom] = y + m.atom_energy[e];
+                            }
+                        }
+                    }
+                __syncwarp();
+            }
+            for (int l = L - 1; l >= 1; --l) {
+                const int wi = m.width[l], wo = m.width[l + 1], NT = (wi + 7) >> 3;
+                const int nb = ((wo + 3) >> 2) * NT * 32;
+                rows_gemm(acc, yrow, wo, h - nb, NT, r, q, lane);
+                h -= nb + ((wi + 3) >> 2) * ((wo + 7) >> 3) * 32;
+                __syncwarp();
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const int col = nt * 8 + 2 * q + v;
+                        if (col < wi) yrow[r * kDS + col] = acc[nt][v] * da[((l - 1) * kDR + r) * kDS + col];
+                    }
+                __syncwarp();
+            }
+            // dE/dG = delta_1 W1, four column tiles (independent chains) at a time
+            double afr[kDH / 4];
+#pragma unroll
+            for (int ks = 0; ks < kDH / 4; ++ks) afr[ks] = (4 * ks + q < H1) ? yrow[r * kDS + 4 * ks + q] : 0.0;
+            __syncwarp();
+            double* drow = b.dEdG + (size_t)(atom >= 0 ? atom : 0) * nsf;
+            for (int nb = 0; nb < NB; nb += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc[u][0] = acc[u][1] = 0.0;
+#pragma unroll
+                for (int ks = 0; ks < kDH / 4; ++ks)
+                    if (ks < KB)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (nb + u < NB) dmma(acc[u], afr[ks], Bw[((nb + u) * KB + ks) * 32]);
+                if (atom >= 0)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int col = (nb + u) * 8 + 2 * q;
+                        if (kVec && col + 1 < nin) {
+                            *reinterpret_cast<double2*>(drow + col) = make_double2(acc[u][0], acc[u][1]);
+                        } else {
+                            if (col < nin) drow[col] = acc[u][0];
+                            if (col + 1 < nin) drow[col + 1] = acc[u][1];
+                        }
+                    }
             }
         }
     }
@@ -312,21 +538,34 @@ void run_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     k_mlp<T><<<tiles, kThreads, smem, s>>>(b, m, maxw);
 }
 
-// The tensor-core form takes networks whose layers are at most kDH wide,
+// The tensor-core forms take networks whose layers are at most kDH wide,
 // with one output and at most 8 layers (dm_ok, set with the fragments at
-// model upload).
+// model upload).  The resident form needs an element's weights to fit in
+// shared memory and enough tiles to keep its warps busy: its time for one
+// tile is long (53 us from 4,500 atoms down, against 19-34 us of the split
+// form).  Measured for 280-25-25-1 networks, split / resident: 83 / 86 us at
+// 18,000 atoms, 137 / 141 at 36,000, 250 / 228 at 71,000; the line lies
+// between the last two.
+constexpr int kResidentTilesPerSm = 36;
+
 int launch_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     if (!m.dm_ok) {
         run_mlp<double>(b, m, s);
         return 1;
     }
-    int maxw = 1;
-    for (int l = 1; l <= m.nlayers; ++l) maxw = maxw > m.width[l] ? maxw : m.width[l];
-    const int S = dmma_stride(maxw);
-    const size_t smem = (size_t)dmma_warp_doubles(m.nlayers, S) * sizeof(double) * kDW;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_mlp_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const long long warps = b.natoms / kDR + m.nel + 1;  // >= the tiles of all elements
-    k_mlp_dmma<<<(unsigned)((warps + kDW - 1) / kDW), 32 * kDW, smem, s>>>(b, m, S);
+    int nin = 0;
+    for (int e = 0; e < m.nel; ++e) nin = nin > m.nin_el[e] ? nin : m.nin_el[e];
+    const size_t rsm = (size_t)dmma_layout(m, nin).total * sizeof(double);
+    const int nsm = device_sm_count();
+    if (rsm <= 227 * 1024 && b.natoms >= nsm * kResidentTilesPerSm * kDR) {
+        auto k = (m.nsf_max & 1) ? k_mlp_resident<false> : k_mlp_resident<true>;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
+        k<<<nsm, 32 * kRW, rsm, s>>>(b, m, nin);
+        return 1;
+    }
+    const size_t smem = (size_t)split_doubles(m) * sizeof(double);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k_mlp_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_mlp_split<<<b.natoms / kDR + m.nel + 1, 32 * kDW, smem, s>>>(b, m);
     return 1;
 }
 

@@ -1,0 +1,69 @@
+"""FP64 network kernels (forward, dE/dG) against the layers in numpy, on the
+symmetry functions the device computed: tiles of 8 atoms that are partly
+filled (one atom, one tile less / plus one atom, elements with fewer atoms
+than a tile), and batches on either side of the line between the per-tile and
+the weights-resident kernel, with rows of even (abx3, 280) and odd (prz, 195)
+length.
+
+Tolerance: eps times the terms of the longest sum times the largest sum of
+absolute products, carried through the later layers by their largest absolute
+row / column sums (activations are 1-Lipschitz)."""
+import numpy as np
+import pytest
+
+from conftest import ABX3_DIR, EXAMPLE_DIR, PRZ_DIR
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(float).eps
+
+
+def layers(net, x):
+    """Energies, dE/dG and their rounding bounds for the rows of x."""
+    ys, ds, grow = [x], [], 1.0
+    scale = 1.0
+    for w, b, a in net:
+        c = ys[-1] @ w.T + b
+        scale = max(scale, (np.abs(ys[-1]) @ np.abs(w).T + np.abs(b)).max())
+        y = np.tanh(c) if a == "t" else np.logaddexp(0.0, c) if a == "p" else np.maximum(c, 0.0) if a == "r" else c
+        d = 1 - y * y if a == "t" else 1 / (1 + np.exp(-c)) if a == "p" else (c > 0) * 1.0 if a == "r" else 1 + 0 * c
+        ys.append(y)
+        ds.append(d)
+        grow *= max(1.0, np.abs(w).sum(1).max(), np.abs(w).sum(0).max()) if len(ys) > 2 else 1.0
+    g = ds[-1]
+    for k in range(len(net) - 1, 0, -1):
+        g = (g @ net[k][0]) * ds[k - 1]
+    tol = 4 * EPS * x.shape[1] * scale * grow
+    return ys[-1][:, 0], g @ net[0][0], tol, tol * max(1.0, np.abs(net[0][0]).max()) * grow
+
+
+@pytest.mark.parametrize("pot_dir, natoms", [(EXAMPLE_DIR, 8), (EXAMPLE_DIR, 1), (ABX3_DIR, 7), (ABX3_DIR, 9),
+                                             (ABX3_DIR, 97), (PRZ_DIR, 65), (ABX3_DIR, 42611), (ABX3_DIR, 42630),
+                                             (PRZ_DIR, 42631)])
+def test_networks(pkg, W, pot_dir, natoms):
+    from hdnnp_b200 import engine
+
+    pot = engine.Hdnnp.from_runner(pot_dir)
+    try:
+        pot.set_option("small_eval", 0)
+        rng = np.random.default_rng(natoms)
+        if pot_dir == EXAMPLE_DIR:
+            s = W.read_xyz(EXAMPLE_DIR + "/input.xyz")
+        else:
+            s = W.supercell(W.abx3_cell(), (17, 15, 14) if natoms > 1000 else (3, 3, 1))
+            s["pos"] = s["pos"] + rng.normal(0, 0.1, s["pos"].shape)
+        Z, pos = s["Z"][:natoms], s["pos"][:natoms]
+        pot.energy_and_forces(engine.AtStruct(Z, pos, s["lat"]))
+        nsf = max(pot.nsf.values())
+        G = pot.fetch("G", natoms * nsf).reshape(natoms, nsf)
+        D = pot.fetch("dEdG", natoms * nsf).reshape(natoms, nsf)
+        E = pot.fetch("atom_energy", natoms)
+        e0 = pot.flags()["atomenergies"]
+        for z in np.unique(Z):
+            m, n = Z == z, pot.nsf[int(z)]
+            e, g, te, tg = layers(pot.network(int(z)), G[m][:, :n])
+            e = e + e0[int(z) - 1]
+            assert np.abs(E[m] - e).max() <= te + 4 * EPS * np.abs(e).max()
+            assert np.abs(D[m][:, :n] - g).max() <= tg
+    finally:
+        pot.close()
