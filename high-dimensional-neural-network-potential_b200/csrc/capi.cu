@@ -197,7 +197,7 @@ struct hdnnp_ctx {
     DevBuf<float> Gf, dEdGf, atEf, gentf, gselff, virf;  // mixed-precision intermediates
     DevBuf<double> cm_acc, cm_E, cm_std;                  // committee: dE/dG sum, member energies, std
     DevBuf<unsigned> pairs;                               // contributing-pair lists (fast kernels)
-    DevBuf<int> npairs;
+    DevBuf<int> npairs, wide;
     DevBuf<int> cnei_cnt, cnei_off, cnei_j, cnei_s, cnei_rev, cnei_map;  // compacted Verlet-skin lists
     DevBuf<int> pad;                                      // padded neighbour rows (int2 pairs)
     DevBuf<double4> posc;                                 // cell-ordered wrapped positions
@@ -255,6 +255,7 @@ struct hdnnp_ctx {
         stats.release();
         pairs.release();
         npairs.release();
+        wide.release();
         for (auto* b : {&cnei_cnt, &cnei_off, &cnei_j, &cnei_s, &cnei_rev, &cnei_map, &pad}) b->release();
         slab.release();
         posc.release();
@@ -411,17 +412,17 @@ int upload_model(hdnnp_model* m) {
                     D.pfz[z] = D.zint[z] >= 0 ? std::ldexp(1.0, -D.zint[z]) : std::pow(2.0, 1.0 - zets[z]);
                 }
                 for (int e = 0; e < D.fe; ++e) D.eta4[e] = etas[e];
-                // integer eta ratios: exp(-eta_e R) = exp(-eta_0 R)^k_e
-                bool ints = D.fe > 1 && etas[0] > 0.0;
-                for (int e = 1; e < D.fe && ints; ++e) {
-                    const double k = etas[e] / etas[0], kr = std::nearbyint(k);
-                    ints = kr >= 2.0 && kr <= 64.0 && std::fabs(k - kr) <= 1e-12 * kr;
-                    D.eta_k[e] = (int)kr;
-                }
-                if (!ints)
-                    for (int e = 0; e < 8; ++e) D.eta_k[e] = 0;
-                else
-                    D.eta_k[0] = 1;
+                D.exp_bounded = 1;
+                for (auto& E : H.el)
+                    for (auto& f : E.sfs) {
+                        const double x = H.max_rc + std::fabs(f.rs);
+                        if (f.type == 2 && !(f.eta >= 0.0 && f.eta * x * x <= 700.0)) D.exp_bounded = 0;
+                    }
+                D.g4_full = 1;
+                for (size_t g = 0; g + 1 < g4_off.size(); ++g)
+                    if (g4_off[g + 1] == g4_off[g]) D.g4_full = 0;
+                for (int e = 0; e < D.fe; ++e)
+                    if (!(etas[e] >= 0.0 && etas[e] * H.max_rc * H.max_rc <= 1.5)) D.exp_bounded = 0;
                 int bit = 0;
                 while ((1 << (bit + 1)) <= maxz) ++bit;
                 D.zmaxbit = bit;
@@ -571,6 +572,14 @@ int upload_model(hdnnp_model* m) {
         if (dmf.empty()) dmf.assign(1, 0.0);
         if (dmb.empty()) dmb.assign(1, 0.0);
     }
+    std::vector<double2> pscale(pmap.size(), double2{0.0, 0.0});
+    for (size_t q = 0; D.fast && q < pmap.size(); ++q) {
+        if (pmap[q] < 0) continue;
+        const int P = fast_shape_p(D.fast), NZ = kFastShapes[D.fast][1], NE = kFastShapes[D.fast][2];
+        const size_t at = q / ((size_t)nblk * P) * nsf_max + pmap[q];
+        pscale[q] = double2{D.pfz[(q % P) / NE % NZ] * sinvw[at], -smean[at] * sinvw[at]};
+    }
+    size_t o_ps = add(pscale.data(), pscale.size() * sizeof(double2));
     size_t o_pm = add(pmap.data(), pmap.size() * sizeof(short)), o_wf = add(wf.data(), wf.size() * 4),
            o_wtf = add(wtf.data(), wtf.size() * 4), o_bf = add(bf.data(), bf.size() * 4),
            o_tcf = add(tcf.data(), tcf.size() * 2), o_tcb = add(tcb.data(), tcb.size() * 2),
@@ -584,6 +593,8 @@ int upload_model(hdnnp_model* m) {
     D.nsf = (const int*)(base + o_nsf);
     D.g2_off = (const int*)(base + o_g2o);
     D.g2max = 0;
+    D.g2el_max = 0;
+    for (size_t g = 0; g + 1 < g2_off.size(); ++g) D.g2el_max = std::max(D.g2el_max, g2_off[g + 1] - g2_off[g]);
     for (int c = 0; c < nel; ++c) D.g2max = std::max(D.g2max, g2_off[(size_t)c * nel + nel] - g2_off[(size_t)c * nel]);
     D.g2 = (const SF2*)(base + o_g2);
     D.g4_off = (const int*)(base + o_g4o);
@@ -598,6 +609,7 @@ int upload_model(hdnnp_model* m) {
     D.b_off = (const long long*)(base + o_bo);
     D.atom_energy = (const double*)(base + o_ae);
     D.pmap = (const short*)(base + o_pm);
+    D.pscale = (const double2*)(base + o_ps);
     D.wf = (const float*)(base + o_wf);
     D.wtf = (const float*)(base + o_wtf);
     D.bf = (const float*)(base + o_bf);
@@ -817,7 +829,10 @@ int run_pipeline(hdnnp_ctx* c, int nstruct, int natoms, const int32_t* Zd, const
     fast = D.fast && !c->generic_sf;
     mixed = c->precision == HDNNP_PREC_MIXED && fast;
     if (fast) {
-        if ((r = c->pairs.ensure(N * (size_t)kPairCap)) || (r = c->npairs.ensure(N))) return r;
+        if ((r = c->pairs.ensure(N * (size_t)kPairCap)) || (r = c->npairs.ensure(N)) ||
+            (r = c->wide.ensure(N + 2)))
+            return r;
+        b.wide = c->wide.p;
         b.pairs = c->pairs.p;
         b.npairs = c->npairs.p;
         b.pcap = kPairCap;

@@ -63,6 +63,7 @@ struct DevModel {
     const int* nsf;           // [nel]
     const int* g2_off;        // [nel*nel+1]
     int g2max;                // most radial SFs of one centre element
+    int g2el_max;             // most radial SFs of one (centre, neighbour) element pair
     const SF2* g2;
     const int* g4_off;        // [nel*nblk+1]
     const SF4* g4;
@@ -92,12 +93,14 @@ struct DevModel {
     int zint[8];              // zeta - 1 if zeta is an integer >= 1, else -1
     double pfz[8];            // 2^(1 - zeta)
     double eta4[8];
-    // eta4[e] / eta4[0] when every ratio is an integer 2..64 (ascending
-    // etas), else 0: the FP64 kernels then take exp(-eta_e R) as
-    // exp(-eta_0 R)^k_e by squaring, one exponential per pair
-    int eta_k[8];
+    // 1 when 0 <= eta rc^2 <= 1.5 for every angular eta and 0 <= eta (rc +
+    // |rs|)^2 <= 700 for every radial function: the FP64 kernels then take
+    // their exponentials without range tests (fastmath.cuh)
+    int exp_bounded;
+    int g4_full;              // 1 when every centre element has angular functions for every element pair
     int zmaxbit;              // highest bit of the integer zeta - 1 values
     const short* pmap;        // [nel][nblk][P]: SF index of product entry p, or -1
+    const double2* pscale;    // [nel][nblk][P]: G = x * sum + y (2^(1-zeta) / width, -mean / width)
     // FP32 copies of the network weights (mixed-precision form)
     const float* wf;
     const float* wtf;
@@ -190,6 +193,10 @@ struct Batch {
     unsigned* pairs;          // [natoms * pcap]
     int* npairs;              // [natoms]
     int pcap;
+    // Atoms with more neighbours than the first launch of a fast pass takes:
+    // [0] and [1] their number in the value and the gradient pass, then the
+    // list (each pass its own, one after the other).
+    int* wide;                // [natoms + 2]
     // Launch shape of the fast symmetry-function kernels (0: defaults): the
     // neighbour count splitting the two launches (-1: one launch) and the
     // persistent grid in blocks per SM.  Set by the plans' autotuner.

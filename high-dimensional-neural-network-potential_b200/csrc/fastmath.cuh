@@ -20,27 +20,19 @@
 //    libm (tests/test_fastmath.py emulates these operations on the host
 //    with exact fused multiply-adds, and checks the device functions, run
 //    through hdnnp_debug_math, against libm's exp, tanh and sqrt).
-//  * tanh01(u) = (1 - e^(-2u)) / (1 + e^(-2u)) with the quotient from the
-//    hardware reciprocal approximation refined by one third-order Newton
-//    step and one residual correction (Newton-Raphson division, as in
-//    P. Markstein, "IA-64 and Elementary Functions", 2000).  Absolute error
-//    a few 1e-16; its relative error grows as u -> 0, where the cutoff
-//    function tanh^3 and its derivative vanish.
+//  * exp_small(x) for x in [-1.5, 0] and tanh01(u) for u in [0, 1]:
+//    polynomials interpolated at Chebyshev nodes (in 60 decimal digits, then
+//    rounded), two Horner chains each; no reduction, no reciprocal.
 //  * sqrt_rsqrt(x) and rsqrt_pos(x): the hardware reciprocal square-root
 //    approximation refined by one third-order Newton step; the root as
 //    x * rsqrt with one residual correction.  x = 0 gives 0 (the reciprocal
 //    is taken of max(x, 1e-300)).
 // The constants are ln 2 and 1/ln 2 rounded to double, the remainder
-// ln 2 - double(ln 2), 1.5 * 2^52 (the round-to-integer shifter) and 1/n!.
+// ln 2 - double(ln 2), 1.5 * 2^52 (the round-to-integer shifter), 1/n! and
+// the interpolants'.
 #pragma once
 
 namespace hdnnp {
-
-__device__ __forceinline__ double rcp_approx(double d) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    return y;
-}
 
 __device__ __forceinline__ double rsqrt_approx(double x) {
     double y;
@@ -78,25 +70,69 @@ __device__ __forceinline__ double exp_clamped(double x) {
     return p * __hiloint2double((k + 1023) << 20, 0);
 }
 
-// 1 / d for d in [1, 2]
-__device__ __forceinline__ double rcp_12(double d) {
-    double y = rcp_approx(d);
-    const double e = fma(-d, y, 1.0);
-    return fma(y, fma(e, e, e), y);  // y (1 + e + e^2)
+// Coefficients, read as constant-bank operands of the multiply-adds: as
+// literals each would cost two moves into registers per use.
+__constant__ double kExpSmall[13] = {0.5, 0.16666666666666613, 0.04166666666664616, 0.008333333333031724,
+                                     0.0013888888865815077, 0.0001984126878917537, 2.4801556448973442e-05,
+                                     2.755671130771333e-06, 2.7549086858331984e-07, 2.4975059697137715e-08,
+                                     2.0384099238823596e-09, 1.39778776896738e-10, 6.046017537551262e-12};
+__constant__ double kTanh01[16] = {1.0, -0.3333333333333273, 0.13333333333282113, -0.05396825395091773,
+                                   0.021869488226930838, -0.008863232181130274, 0.003592104115230281,
+                                   -0.00145571559077928, 0.0005896028950856166, -0.00023801236323479905,
+                                   9.472256075732066e-05, -3.603918536997382e-05, 1.2306805295349983e-05,
+                                   -3.402993826979274e-06, 6.496857637862531e-07, -6.20675330545365e-08};
+
+// e^x for x in [-1.5, 0]: 1 + x + x^2 q(x), q the degree-12 Chebyshev
+// interpolant of (e^x - 1 - x) / x^2 on the interval (error 1e-16)
+__device__ __forceinline__ double exp_small(double x) {
+    const double x2 = x * x;
+    double a = kExpSmall[12], b = kExpSmall[11];
+#pragma unroll
+    for (int k = 10; k >= 0; k -= 2) a = fma(a, x2, kExpSmall[k]);
+#pragma unroll
+    for (int k = 9; k >= 1; k -= 2) b = fma(b, x2, kExpSmall[k]);
+    return 1.0 + fma(fma(b, x, a), x2, x);
 }
 
-// tanh(u) for u in [0, 1]
+// tanh(u) for u in [0, 1]: u p(u^2), p the degree-15 Chebyshev interpolant of
+// tanh(sqrt v) / sqrt v on [0, 1] (error 6e-17)
 __device__ __forceinline__ double tanh01(double u) {
-    const double t = exp_clamped(-2.0 * u);
-    const double n = 1.0 - t, d = 1.0 + t;
-    const double y = rcp_12(d);
-    const double q = n * y;
-    return fma(y, fma(-d, q, n), q);
+    const double v = u * u, w = v * v;
+    double a = kTanh01[14], b = kTanh01[15];
+#pragma unroll
+    for (int k = 12; k >= 0; k -= 2) a = fma(a, w, kTanh01[k]);
+#pragma unroll
+    for (int k = 13; k >= 1; k -= 2) b = fma(b, w, kTanh01[k]);
+    return u * fma(b, v, a);
+}
+
+// e^x for x in [-700, 0], the operations of exp_clamped without the range
+// clamp and with its coefficients in the constant bank
+__constant__ double kExpNeg[16] = {1.4426950408889634, 6755399441055744.0, 0.6931471805599453, 2.3190468138462996e-17,
+                                   0.5, 0.16666666666666666, 0.041666666666666664, 0.008333333333333333,
+                                   0.001388888888888889, 0.0001984126984126984, 2.48015873015873e-05,
+                                   2.7557319223985893e-06, 2.755731922398589e-07, 2.505210838544172e-08,
+                                   2.08767569878681e-09, 1.6059043836821613e-10};
+__device__ __forceinline__ double exp_neg(double x) {
+    const double t = fma(x, kExpNeg[0], kExpNeg[1]);
+    const int k = __double2loint(t);
+    const double kd = t - kExpNeg[1];
+    double r = fma(kd, -kExpNeg[2], x);
+    r = fma(kd, -kExpNeg[3], r);
+    const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4;
+    const double q1 = fma(kExpNeg[5], r, kExpNeg[4]), q2 = fma(kExpNeg[7], r, kExpNeg[6]);
+    const double q3 = fma(kExpNeg[9], r, kExpNeg[8]), q4 = fma(kExpNeg[11], r, kExpNeg[10]);
+    const double q5 = fma(kExpNeg[13], r, kExpNeg[12]), q6 = fma(kExpNeg[15], r, kExpNeg[14]);
+    const double s0 = fma(q1, r2, r), s1 = fma(q3, r2, q2), s2 = fma(q5, r2, q4);
+    const double t0 = fma(s1, r4, s0), t1 = fma(q6, r4, s2);
+    const double p = 1.0 + fma(t1, r8, t0);
+    return p * __hiloint2double((k + 1023) << 20, 0);
 }
 
 // 1 / sqrt(x) for x > 0 (x = 0 gives 1e150)
 __device__ __forceinline__ double rsqrt_pos(double x) {
-    const double xc = fmax(x, 1e-300);
+    // max(x, 1e-300) on the high word (x >= 0; the low word only matters above)
+    const double xc = __hiloint2double(max(__double2hiint(x), 0x01a56e1f), __double2loint(x));
     const double y = rsqrt_approx(xc);
     const double e = fma(-xc * y, y, 1.0);                     // 1 - x y^2
     return fma(y * e, fma(0.375, e, 0.5), y);                  // y (1 + e/2 + 3e^2/8)

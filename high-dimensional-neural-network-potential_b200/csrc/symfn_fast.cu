@@ -4,21 +4,22 @@
 // Same mathematics as symfn.cu (calcAllSymmetryFunctions,
 // symmetryFunctions.f90:158-308; scaling hdnnps.f90:471-481), organised so
 // that the per-(pair, SF) work is one fused multiply-add:
-//   * per pair: X_l = 1 + lambda_l cos, one square chain X, X^2, X^4, ...
-//     shared by every zeta, T_lz = X_l^zeta_z (and X_l^(zeta_z - 1) for the
-//     gradient), and one exponential Y_e = exp(-eta_e (r_ij^2+r_ik^2+r_jk^2))
-//     per distinct eta;
-//   * pass 1 accumulates acc[l,z,e] += T_lz Y_e fcp in registers and maps the
-//     product entries to SF indices at the end of each element-pair block
-//     (G_s = 2^(1-zeta) acc[l,z,e]);
-//   * pass 2 stages per block the weight tensors WA[l,z,e] = w_s 2^(1-zeta)
-//     and WC = WA lambda zeta (w_s = dE/dG_s / (max_s - min_s)) and contracts
-//     A = sum WA T Y, B = sum eta WA T Y, C = sum WC T' Y per pair, from which
-//     dE/dr_j and dE/dr_k are assembled as in symfn.cu.
-// Per-neighbour 1/r is precomputed, so a pair needs one sqrt, one tanh and
-// one exp per distinct eta.  Warp per centre atom; neighbours staged in
-// shared memory sorted by element; candidate pairs compacted through a shared
-// queue; chunks of 32 contributing pairs, one per lane.
+//   * per neighbour (staging): everything that depends on it alone, 1/r and
+//     P_e = fc exp(-eta_e r^2) for every distinct eta;
+//   * per pair: cos from the three squared distances, X_l = 1 + lambda_l cos,
+//     one square chain X, X^2, X^4, ... shared by every zeta, T_lz =
+//     X_l^zeta_z (and X_l^(zeta_z - 1) for the gradient), fc(r_jk) and one
+//     exp(-eta_e r_jk^2) per eta;
+//   * pass 1 adds acc[l,z,e] += T_lz Y_e, Y_e = P_je P_ke exp(-eta_e r_jk^2)
+//     fc(r_jk), on the FP64 tensor cores and maps the product entries to SF
+//     indices (G_s = 2^(1-zeta) acc[l,z,e]);
+//   * pass 2 stages per element-pair block the weight tensor WA[l,z,e] = w_s
+//     2^(1-zeta) (w_s = dE/dG_s / (max_s - min_s)), contracts it with the
+//     powers and their derivatives, and takes dE/dr_j and dE/dr_k from the
+//     derivatives with respect to r_ij^2, r_ik^2 and r_jk^2.
+// A warp per centre atom; neighbours staged in shared memory sorted by
+// element; the contributing pairs (r_jk < rc) compacted into lists of which a
+// chunk of 32 is evaluated at a time, one pair per lane.
 #include <algorithm>
 
 #include "engine.h"
@@ -30,10 +31,18 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarps = 4;
-// Resident blocks per SM the FP32 kernels are compiled for (registers): 7 x 4
-// warps for the value pass, 8 x 4 for the gradient pass (a few bytes of
-// spill), which the shared memory of a launch sized for 64 neighbours also
-// allows.  The FP64 kernels keep their registers (4 blocks).
+// parts of a pass: one launch for all atoms, or one for those with few
+// neighbours, which lists the others, and one for the listed
+constexpr int kPartAll = 0, kPartFirst = 1, kPartWide = 2;
+// Resident blocks per SM that the kernels are compiled for (registers) and
+// the default split of a pass is sized for (shared memory): value pass 5 FP64
+// (96 registers) and 6 FP32; gradient pass 4 FP64 (122 registers, no spills;
+// at 5 its four accumulator copies leave 44 neighbours and the pass takes
+// 5.4 ms instead of 3.6 on 1024 structures) and 7 FP32.
+template <typename T>
+constexpr int kBlocksV = sizeof(T) == 4 ? 6 : 5;
+template <typename T>
+constexpr int kBlocksG = sizeof(T) == 4 ? 7 : 4;
 
 template <typename T>
 struct alignas(4 * sizeof(T)) V4 {
@@ -42,37 +51,94 @@ struct alignas(4 * sizeof(T)) V4 {
 
 __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~size_t(15); }
 
-template <typename T>
-struct FSmem {
-    V4<T>* nb;      // dx, dy, dz, r        (centre - neighbour)
-    double4* dd;    // FP32 value pass: the FP64 relative vector (x, y, z, -) for the pair cutoff
-    V4<T>* ax;      // fc, dfc/r, 1/r, -
-    T* gx;          // gradient accumulators (pass 2), one array per component:
-    T* gy;          // a slot's x, y, z in one 16- or 32-byte record put random
-    T* gz;          // slots on 4 (FP64) or 8 (FP32) bank groups only
-    int* ent;       // entry index of a slot (pass 2)
-    unsigned char* el;
-    unsigned* queue;
-    int* est;
-    int* cur;
-    T* w2;          // dE/dG / width of the centre's radial SFs (pass 2)
-    T* WA;          // [nblk][P] (pass 2)
-    T* WC;
-    T* red;         // [32][P+1] (pass 1)
+// ---------------------------------------------------------------- grid specs
+// Spec<NL, NZ, NE, Z0..Z3>: compiled shape of the lambda x zeta x eta grid.
+// With Z0 > 0 the zeta values are compile-time constants (the power chain and
+// every product are straight-line code); with Z0 == 0 they are read from the
+// model (uniform branches).
+template <int NL_, int NZ_, int NE_, int Z0 = 0, int Z1 = 0, int Z2 = 0, int Z3 = 0>
+struct Spec {
+    static constexpr int NL = NL_, NZ = NZ_, NE = NE_, P = NL_ * NZ_ * NE_;
+    static constexpr bool kFixed = Z0 > 0;
+    __host__ __device__ static constexpr int zeta(int z) { return z == 0 ? Z0 : z == 1 ? Z1 : z == 2 ? Z2 : Z3; }
+    __host__ __device__ static constexpr int maxbit() {
+        int mz = 1;
+        for (int z = 0; z < NZ_; ++z) mz = zeta(z) > mz ? zeta(z) : mz;
+        int b = 0;
+        while ((1 << (b + 1)) <= mz) ++b;
+        return b;
+    }
 };
 
+template <class S>
+__device__ __forceinline__ double zeta_of(const DevModel& m, int z) {
+    return S::kFixed ? (double)S::zeta(z) : m.zet[z];
+}
+
+template <class S>
+__device__ __forceinline__ int n_eta(const DevModel& m) {
+    return S::kFixed ? S::NE : m.fe;
+}
+
+// values per neighbour in FSmem::ax: 1/r, rank of the element (value pass,
+// an integer in the low bits) or rho (gradient pass) and P_e = fc exp(-eta_e r^2) of every eta, padded to whole vectors
+template <class S>
+constexpr int kAx = (S::NE + 3) & ~1;
+// rows and row stride of the value pass's term buffer (tensor-core A rows)
+template <class S>
+constexpr int kTRows = ((S::NL * S::NZ + 7) / 8) * 8;
+constexpr int kTs = 36;
+// row stride of the gradient pass's weight tensors: rows of different blocks
+// on different banks (lanes of a chunk read several)
+template <class S>
+constexpr int kWp = S::P + 4;
+
+// copies of the gradient accumulators, one per group of 32 / kCopies lanes
+constexpr int kCopies = 4;
+
 template <typename T>
-__host__ __device__ inline size_t fast_warp_bytes(int mm, int g2max, int nblk, int P, bool grad) {
-    size_t b = a16(sizeof(V4<T>) * mm) * 2;
-    if (sizeof(T) == 4 && !grad) b += a16(sizeof(double4) * mm);
-    if (grad) b += 3 * a16(sizeof(T) * mm) + a16(sizeof(int) * mm) + a16(sizeof(T) * g2max) + 2 * a16(sizeof(T) * nblk * P);
-    else b += a16(sizeof(T) * 32 * (P + 1));
-    b += a16(mm) + 64 * sizeof(unsigned) + a16(sizeof(int) * (kMaxEl + 1)) + a16(sizeof(int) * kMaxEl);
+struct FSmem {
+    V4<T>* nb;      // dx, dy, dz, r^2      (centre - neighbour)
+    double4* dd;    // FP32 value pass: the FP64 relative vector (x, y, z, -) for the pair cutoff
+    float4* sp;     // FP64 value pass: FP32 copy of the relative vector for the candidate test
+    T* rf;          // value pass: r and fc for the radial functions; sp takes the place afterwards
+    T* ax;          // [mm][kAx] per-neighbour factors
+    T* gx;          // gradient accumulators (pass 2): kCopies copies of an array
+    int gst;        // per component, gst values apart (a slot's x, y, z in one
+                    // 16- or 32-byte record put random slots on 4 (FP64) or 8
+                    // (FP32) bank groups only)
+    int* ent;       // entry index of a slot (pass 2)
+    unsigned* queue;  // contributing pairs j | k << 10 (pass 1: kListCap or more; pass 2: ring of 64 with the block)
+    unsigned* mask;   // [mm/32][32] contributing neighbours k > j of the rows j of a batch (pass 1)
+    unsigned char* tm;  // [nel][nel] element-pair block of two ranks, 255: no functions (pass 1)
+    int* est;         // first slot of an element
+    int* cnt;         // its slots
+    int* rst;         // first slot of a rank, [nel + 1]
+    int* ord;         // element of a rank
+    T* w2;          // dE/dG / width of the centre's radial SFs (pass 2)
+    T* WA;          // [nblk][P] (pass 2)
+    T* tb;          // [kTRows][kTs] powers of a chunk's pairs (pass 1)
+    T* yb;          // [8 columns][kTs] their exponential and cutoff factors, zero between uses (pass 1)
+};
+
+__host__ __device__ inline int mask_words(int mm) { return (mm + 31) / 32 * 32; }
+// pairs the value pass lists at a time: a row (one neighbour's pairs) and a
+// chunk's remainder always fit
+constexpr int kListCap = 160;
+__host__ __device__ inline int list_cap(int mm) { return mm + 32 > kListCap ? mm + 32 : kListCap; }
+
+template <typename T, class S>
+__host__ __device__ inline size_t fast_warp_bytes(int mm, int nel, int g2max, int nblk, bool grad) {
+    size_t b = a16(sizeof(V4<T>) * mm) + a16(sizeof(T) * kAx<S> * mm);
+    if (grad) b += kCopies * 3 * a16(sizeof(T) * mm) + a16(sizeof(int) * mm) + a16(sizeof(T) * g2max) + a16(sizeof(T) * nblk * kWp<S>);
+    else b += (sizeof(T) == 4 ? a16(sizeof(double4) * mm) : 0) + a16(2 * sizeof(T) * mm) +
+              (kTRows<S> + 8) * kTs * sizeof(T) + a16(sizeof(unsigned) * mask_words(mm)) + a16(nel * nel);
+    b += a16(sizeof(unsigned) * (grad ? 64 : list_cap(mm))) + 3 * a16(sizeof(int) * kMaxEl) + a16(sizeof(int) * (kMaxEl + 1));
     return b;
 }
 
-template <typename T>
-__device__ inline FSmem<T> fcarve(unsigned char* p, int mm, int g2max, int nblk, int P, bool grad) {
+template <typename T, class S>
+__device__ inline FSmem<T> fcarve(unsigned char* p, int mm, int nel, int g2max, int nblk, bool grad) {
     FSmem<T> s{};
     auto take = [&](size_t bytes) {
         unsigned char* q = p;
@@ -80,24 +146,51 @@ __device__ inline FSmem<T> fcarve(unsigned char* p, int mm, int g2max, int nblk,
         return q;
     };
     s.nb = (V4<T>*)take(sizeof(V4<T>) * mm);
-    s.dd = (sizeof(T) == 4 && !grad) ? (double4*)take(sizeof(double4) * mm) : nullptr;
-    s.ax = (V4<T>*)take(sizeof(V4<T>) * mm);
+    s.ax = (T*)take(sizeof(T) * kAx<S> * mm);
     if (grad) {
-        s.gx = (T*)take(sizeof(T) * mm);
-        s.gy = (T*)take(sizeof(T) * mm);
-        s.gz = (T*)take(sizeof(T) * mm);
+        s.gx = (T*)take(kCopies * 3 * a16(sizeof(T) * mm));
+        s.gst = (int)(a16(sizeof(T) * mm) / sizeof(T));
         s.ent = (int*)take(sizeof(int) * mm);
         s.w2 = (T*)take(sizeof(T) * g2max);
-        s.WA = (T*)take(sizeof(T) * nblk * P);
-        s.WC = (T*)take(sizeof(T) * nblk * P);
+        s.WA = (T*)take(sizeof(T) * nblk * kWp<S>);
     } else {
-        s.red = (T*)take(sizeof(T) * 32 * (P + 1));
+        if (sizeof(T) == 4) s.dd = (double4*)take(sizeof(double4) * mm);
+        s.rf = (T*)take(2 * sizeof(T) * mm);
+        s.sp = (float4*)s.rf;
+        s.tb = (T*)take(kTRows<S> * kTs * sizeof(T));
+        s.yb = (T*)take(8 * kTs * sizeof(T));
+        s.mask = (unsigned*)take(sizeof(unsigned) * mask_words(mm));
+        s.tm = (unsigned char*)take(nel * nel);
     }
-    s.el = (unsigned char*)take(mm);
-    s.queue = (unsigned*)take(64 * sizeof(unsigned));
-    s.est = (int*)take(sizeof(int) * (kMaxEl + 1));
-    s.cur = (int*)take(sizeof(int) * kMaxEl);
+    s.queue = (unsigned*)take(sizeof(unsigned) * (grad ? 64 : list_cap(mm)));
+    s.est = (int*)take(sizeof(int) * kMaxEl);
+    s.cnt = (int*)take(sizeof(int) * kMaxEl);
+    s.rst = (int*)take(sizeof(int) * (kMaxEl + 1));
+    s.ord = (int*)take(sizeof(int) * kMaxEl);
     return s;
+}
+
+// one neighbour's factors (kAx of them) in 16- or 8-byte loads
+template <int A, typename T>
+__device__ __forceinline__ void ldax(const T* ax, int slot, T (&v)[A]) {
+    if constexpr (A % 4 == 0 && sizeof(T) == 4) {
+#pragma unroll
+        for (int q = 0; q < A / 4; ++q) {
+            const float4 x = reinterpret_cast<const float4*>(ax + slot * A)[q];
+            v[4 * q] = x.x;
+            v[4 * q + 1] = x.y;
+            v[4 * q + 2] = x.z;
+            v[4 * q + 3] = x.w;
+        }
+    } else {
+        struct alignas(2 * sizeof(T)) V2 { T x, y; };
+#pragma unroll
+        for (int q = 0; q < A / 2; ++q) {
+            const V2 x = reinterpret_cast<const V2*>(ax + slot * A)[q];
+            v[2 * q] = x.x;
+            v[2 * q + 1] = x.y;
+        }
+    }
 }
 
 // P consecutive weights of one block from shared memory in 16-byte loads
@@ -157,40 +250,27 @@ __device__ __forceinline__ float xexp(float x) { return __expf(x); }
 __device__ __forceinline__ double xtanh(double x) { return tanh01(x); }
 __device__ __forceinline__ float xtanh(float x) { return tanhf(x); }
 __device__ __forceinline__ double xpow(double x, double y) { return pow(x, y); }
-__device__ __forceinline__ float xpow(float x, float y) { return powf(x, y); }
 
-// Y[e] = exp(-eta_e R) for the distinct etas of the grid (zero beyond ne).
-// kPowers (FP64 with integer eta ratios k_e = eta_e / eta_0,
-// DevModel::eta_k): one exponential and Y[e] = Y[0]^k_e by squaring
-// (relative error about k_e ulp, far below the FP64 tolerances); otherwise
-// one exponential per eta.  With the branch-free FP64 exponential the value
-// pass is faster with one exponential per eta (19.29 against 19.80 ms per C4
-// step: independent sequences instead of a dependent chain of products), the
-// gradient pass with the powers (18.20 against 18.60: it spills at 96
-// registers otherwise).
-template <int NE, bool kPowers, typename T>
-__device__ __forceinline__ void eta_exps(const DevModel& m, int ne, T R, T (&Y)[NE]) {
-    if (kPowers && sizeof(T) == 8 && NE > 1 && m.eta_k[0] == 1) {
-        const T y0 = xexp(-(T)m.eta4[0] * R);
-        Y[0] = y0;
+// exp of an angular -eta r^2 and of a radial -eta (r - rs)^2.  kB: every
+// argument of the potential's functions is in the range of the functions
+// without range tests (DevModel::exp_bounded); a template parameter, so that
+// only one form is in a kernel's code.
+template <bool kB>
+__device__ __forceinline__ double ang_exp(double x) { return kB ? exp_small(x) : exp_clamped(x); }
+template <bool kB>
+__device__ __forceinline__ float ang_exp(float x) { return xexp(x); }
+template <bool kB>
+__device__ __forceinline__ double rad_exp(double x) { return kB ? exp_neg(x) : exp_clamped(x); }
+template <bool kB>
+__device__ __forceinline__ float rad_exp(float x) { return xexp(x); }
+
+// E[e] = exp(-eta_e s) of a pair's r_jk^2 = s for the distinct etas of the
+// grid (zero beyond ne).  kB (DevModel::exp_bounded): FP64 without range
+// reduction.
+template <int NE, bool kB, typename T>
+__device__ __forceinline__ void eta_exps(const DevModel& m, int ne, T s, T (&E)[NE]) {
 #pragma unroll
-        for (int e = 1; e < NE; ++e) {
-            T r = (T)1, base = y0;
-            int k = e < ne ? m.eta_k[e] : 0;
-            if (e >= ne) r = (T)0;
-#pragma unroll
-            for (int bit = 0; bit < 7; ++bit) {
-                if (k & 1) r *= base;
-                k >>= 1;
-                if (!k) break;
-                base *= base;
-            }
-            Y[e] = r;
-        }
-        return;
-    }
-#pragma unroll
-    for (int e = 0; e < NE; ++e) Y[e] = e < ne ? xexp(-(T)m.eta4[e] * R) : (T)0;
+    for (int e = 0; e < NE; ++e) E[e] = e < ne ? ang_exp<kB>(-(T)m.eta4[e] * s) : (T)0;
 }
 
 template <typename T> struct Buf;
@@ -224,21 +304,36 @@ __device__ __forceinline__ void entry_vec(const Batch& b, const StructInfo& S, d
     dz = zi - (b.wpos[3 * j + 2] + lz);
 }
 
+// a rank carried in a T
+template <typename T>
+__device__ __forceinline__ T rank_bits(int r) {
+    if constexpr (sizeof(T) == 8) return __hiloint2double(0, r);
+    else return __int_as_float(r);
+}
+__device__ __forceinline__ int rank_of(double x) { return __double2loint(x); }
+__device__ __forceinline__ int rank_of(float x) { return __float_as_int(x); }
+
 // Stage the neighbour entries of atom i sorted by element (stable).  The
 // relative vectors are formed in FP64 from the wrapped positions and image
 // shifts and then rounded to T.  With a Verlet-skin list (list cutoff above
 // rc) only entries with r < rc are staged; the gradient pass writes zero
 // gradients for the others.  Returns the number of staged entries.
-template <typename T, bool kGrad>
+//
+// Per neighbour, every factor of the angular terms that depends on it alone
+// is formed here, so that a pair evaluates only functions of r_jk:
+//   exp(-eta (r_ij^2 + r_ik^2 + r_jk^2)) fc_ij fc_ik fc_jk
+//     = P_j P_k exp(-eta r_jk^2) fc_jk,       P = fc exp(-eta r^2),
+//   rho = d ln fc / d(r^2) = -3 (1 - t^2) / (2 rc r t), t = tanh(1 - r/rc).
+template <typename T, class S, bool kGrad, bool kB>
 __device__ int fstage(const Batch& b, const DevModel& m, int i, int c, FSmem<T>& s, int lane, int M) {
     const int e0 = b.nei_off[i];
     const int nel = m.nel;
     const double xi = b.wpos[3 * i], yi = b.wpos[3 * i + 1], zi = b.wpos[3 * i + 2];
-    const StructInfo& S = b.info[b.sid[i]];
-    const double rc = m.rc[c];
+    const StructInfo& si = b.info[b.sid[i]];
+    const double rc = m.rc[c], irc = 1.0 / rc;
     const bool filt = b.rc_list > rc;
     const double rc2 = rc * rc;
-    if (lane < nel) s.cur[lane] = 0;
+    if (lane < nel) s.cnt[lane] = 0;
     __syncwarp();
     for (int base = 0; base < M; base += 32) {
         const int q = base + lane;
@@ -249,27 +344,53 @@ __device__ int fstage(const Batch& b, const DevModel& m, int i, int c, FSmem<T>&
             el = b.elem[j];
             if (filt) {
                 double dx, dy, dz;
-                entry_vec(b, S, xi, yi, zi, j, b.nei_s[e0 + q], dx, dy, dz);
+                entry_vec(b, si, xi, yi, zi, j, b.nei_s[e0 + q], dx, dy, dz);
                 keep = dx * dx + dy * dy + dz * dz < rc2;
             }
         }
         const unsigned act = __ballot_sync(kFull, keep);
         if (keep) {
             const unsigned peers = __match_any_sync(act, el);
-            if ((peers & lanemask_lt()) == 0) s.cur[el] += __popc(peers);
+            if ((peers & lanemask_lt()) == 0) s.cnt[el] += __popc(peers);
         }
         __syncwarp();
     }
-    if (lane == 0) {
-        int acc = 0;
+    // elements in ascending order of their counts: the first rows of the
+    // angular pass, which meet every element, are few
+    int total;
+    {
+        const int n = lane < nel ? s.cnt[lane] : 0;
+        int rank = 0, start = 0;
+        total = 0;
         for (int x = 0; x < nel; ++x) {
-            s.est[x] = acc;
-            acc += s.cur[x];
+            const int nx = __shfl_sync(kFull, n, x);
+            total += nx;
+            if (nx < n || (nx == n && x < lane)) {
+                ++rank;
+                start += nx;
+            }
         }
-        s.est[nel] = acc;
+        if (lane < nel) {
+            s.est[lane] = start;
+            s.rst[rank] = start;
+            s.ord[rank] = lane;
+        }
+        if (lane == 0) s.rst[nel] = total;
+        __syncwarp();
+        if (!kGrad) {
+            const int mine = lane < nel ? s.ord[lane] : 0;
+            for (int q = 0; q < nel; ++q) {
+                const int other = __shfl_sync(kFull, mine, q);
+                if (lane < nel) {
+                    const int lo = min(mine, other), hi = max(mine, other);
+                    const int t = lo * nel - lo * (lo - 1) / 2 + hi - lo;
+                    const bool has = m.g4_full || m.g4_off[c * m.nblk + t + 1] > m.g4_off[c * m.nblk + t];
+                    s.tm[lane * nel + q] = has ? (unsigned char)t : (unsigned char)255;
+                }
+            }
+        }
     }
-    __syncwarp();
-    if (lane < nel) s.cur[lane] = s.est[lane];
+    // est moves while slots are handed out and is set back below
     __syncwarp();
     for (int base = 0; base < M; base += 32) {
         const int q = base + lane;
@@ -280,7 +401,7 @@ __device__ int fstage(const Batch& b, const DevModel& m, int i, int c, FSmem<T>&
             j = b.nei_j[e0 + q];
             sh = b.nei_s[e0 + q];
             el = b.elem[j];
-            entry_vec(b, S, xi, yi, zi, j, sh, dx, dy, dz);
+            entry_vec(b, si, xi, yi, zi, j, sh, dx, dy, dz);
             if (filt && !(dx * dx + dy * dy + dz * dz < rc2)) {
                 keep = false;
                 if (kGrad) {
@@ -295,59 +416,106 @@ __device__ int fstage(const Batch& b, const DevModel& m, int i, int c, FSmem<T>&
         const unsigned act = __ballot_sync(kFull, keep);
         if (keep) {
             const unsigned peers = __match_any_sync(act, el);
-            slot = s.cur[el] + __popc(peers & lanemask_lt());
+            slot = s.est[el] + __popc(peers & lanemask_lt());
             __syncwarp(act);
-            if ((peers & lanemask_lt()) == 0) s.cur[el] += __popc(peers);
+            if ((peers & lanemask_lt()) == 0) s.est[el] += __popc(peers);
         }
         __syncwarp();
         if (keep) {
-            // distance and cutoff in FP64
+            // distance, cutoff and exponentials in FP64
+            const double r2 = dx * dx + dy * dy + dz * dz;
             double r, ir;
-            sqrt_rsqrt(dx * dx + dy * dy + dz * dz, r, ir);
-            const double irc = 1.0 / rc;
-            double fc = 0.0, dfc = 0.0;
+            sqrt_rsqrt(r2, r, ir);
+            double fc = 0.0, rho = 0.0;
             if (r < rc) {
                 const double t = tanh01(1.0 - r * irc), tt = t * t;
                 fc = tt * t;
-                dfc = -3.0 * irc * ir * (tt - tt * tt);
+                if (kGrad && t > 0.0) rho = -1.5 * irc * ir * (1.0 - tt) / t;
             }
-            s.nb[slot] = V4<T>{(T)dx, (T)dy, (T)dz, (T)r};
-            if (sizeof(T) == 4 && s.dd)
-                s.dd[slot] = make_double4(dx, dy, dz, 0.0);
-            s.ax[slot] = V4<T>{(T)fc, (T)dfc, (T)ir, (T)0};
-            s.el[slot] = (unsigned char)el;
+            s.nb[slot] = V4<T>{(T)dx, (T)dy, (T)dz, (T)r2};
+            T* ax = s.ax + slot * kAx<S>;
+            ax[0] = (T)ir;
+            if (kGrad) ax[1] = (T)rho;
+#pragma unroll
+            for (int e = 0; e < S::NE; ++e)
+                ax[2 + e] = e < n_eta<S>(m)
+                                ? (T)(fc * ang_exp<kB>(-m.eta4[e] * r2))
+                                : (T)0;
             if (kGrad) {
-                s.gx[slot] = s.gy[slot] = s.gz[slot] = (T)0;
+                // r, fc and the element wait in the accumulators for the
+                // radial pass, which starts the sums
+                s.gx[slot] = (T)r;
+                s.gx[s.gst + slot] = (T)fc;
+                s.gx[2 * s.gst + slot] = (T)el;
                 s.ent[slot] = e0 + q;
+            } else {
+                if (sizeof(T) == 4) s.dd[slot] = make_double4(dx, dy, dz, 0.0);
+                s.rf[2 * slot] = (T)r;
+                s.rf[2 * slot + 1] = (T)fc;
             }
         }
     }
     __syncwarp();
-    return s.est[nel];
+    if (lane < nel) s.est[lane] -= s.cnt[lane];
+    __syncwarp();
+    if (!kGrad) {
+        for (int q = lane; q < total; q += 32) {
+            int rank = 0;
+            for (int x = 1; x < nel; ++x) rank += q >= s.rst[x];
+            s.ax[q * kAx<S> + 1] = rank_bits<T>(rank);
+        }
+        __syncwarp();
+    }
+    return total;
 }
 
-// Candidate c of block (a,b) -> slots (j,k) without divisions: rectangular
-// blocks use a float reciprocal of nb (exact for these sizes), triangular
-// blocks a float square root with integer fix-ups.
-__device__ __forceinline__ void fpair(int c, int sa, int na, int sb, int nb, bool same, float inv_nb, int& j, int& k) {
-    if (!same) {
-        int jj = (int)(((float)c + 0.5f) * inv_nb);
-        int kk = c - jj * nb;
-        if (kk < 0) { --jj; kk += nb; }
-        else if (kk >= nb) { ++jj; kk -= nb; }
-        j = sa + jj;
-        k = sb + kk;
-    } else {
-        const float t = (float)(2 * na - 1);
-        int jj = (int)((t - sqrtf(fmaxf(t * t - 8.0f * (float)c, 0.0f))) * 0.5f);
-        if (jj < 0) jj = 0;
-        auto off = [&](int x) { return x * (2 * na - x - 1) / 2; };
-        while (jj > 0 && off(jj) > c) --jj;
-        while (off(jj + 1) <= c) ++jj;
-        j = sa + jj;
-        k = sa + jj + 1 + (c - off(jj));
+// Candidate pairs of one element-pair block, 32 at a time: lane L holds the
+// candidates L, L + 32, ... of na rows (neighbours of element a) times W
+// columns.  Different elements: every neighbour of b.  Equal elements: row x
+// pairs with the next W = na/2 neighbours in cyclic order, which meets every
+// unordered pair once (for even na the last column holds each of its pairs
+// twice, and its second half of rows is left out).  Stepping needs no
+// division and no square root per candidate.
+struct PairRows {
+    int sa, sb, na, W, ncand;
+    int row, col, qs, rs;
+    bool same, even;
+    __device__ __forceinline__ void start(int sa_, int na_, int sb_, int nb_, bool same_, bool has, int lane) {
+        sa = sa_;
+        sb = sb_;
+        na = na_;
+        same = same_;
+        even = same && !(na & 1);
+        W = has ? (same ? na >> 1 : nb_) : 0;
+        ncand = na * W;
+        const float inv = ncand > 0 ? 1.0f / (float)W : 0.0f;
+        row = (int)(((float)lane + 0.5f) * inv);
+        col = lane - row * W;
+        qs = (int)(32.5f * inv);
+        rs = 32 - qs * W;
     }
-}
+    // the lane's candidate, if it has one in this chunk
+    __device__ __forceinline__ bool get(int& j, int& k) const {
+        j = sa + row;
+        int kk = sb + col;
+        bool ok = row < na && ncand > 0;
+        if (same) {
+            kk = row + 1 + col;
+            kk = sa + (kk >= na ? kk - na : kk);
+            ok = ok && !(even && col == W - 1 && row >= W);
+        }
+        k = kk;
+        return ok;
+    }
+    __device__ __forceinline__ void next() {
+        row += qs;
+        col += rs;
+        if (col >= W) {
+            col -= W;
+            ++row;
+        }
+    }
+};
 
 // u = 1 - r_jk/rc for the pair cutoff.  In the FP32 form the difference
 // cancels near rc; it is formed as (rc^2 - r_jk^2) / (rc (rc + r_jk)) with
@@ -356,8 +524,7 @@ __device__ __forceinline__ void fpair(int c, int sa, int na, int sb, int nb, boo
 // inside rc (whose SFs can have tiny scaling ranges and therefore large
 // weights).  The gradient pass takes it from the FP32 vectors: its terms of
 // such pairs scale with u^2, so the absolute error stays at FP32 rounding,
-// and leaving the FP64 vectors out of its shared memory lets 8 blocks of it
-// reside per SM instead of 7 (13.7 -> 11.3 ms per C4 step).
+// and the FP64 vectors stay out of its shared memory.
 template <typename T>
 __device__ __forceinline__ T pair_u(const FSmem<T>& s, int j, int k, double rc2d, T rc, T inv_rc, T rjk) {
     if (sizeof(T) == 8) {
@@ -384,25 +551,7 @@ __device__ __forceinline__ T pair_u(const FSmem<T>& s, int j, int k, double rc2d
     return D > 0.0 ? xdiv((T)D, rc * (rc + rjk)) : (T)0;
 }
 
-// ---------------------------------------------------------------- grid specs
-// Spec<NL, NZ, NE, Z0..Z3>: compiled shape of the lambda x zeta x eta grid.
-// With Z0 > 0 the zeta values are compile-time constants (the power chain and
-// every product are straight-line code); with Z0 == 0 they are read from the
-// model (uniform branches).
-template <int NL_, int NZ_, int NE_, int Z0 = 0, int Z1 = 0, int Z2 = 0, int Z3 = 0>
-struct Spec {
-    static constexpr int NL = NL_, NZ = NZ_, NE = NE_, P = NL_ * NZ_ * NE_;
-    static constexpr bool kFixed = Z0 > 0;
-    __host__ __device__ static constexpr int zeta(int z) { return z == 0 ? Z0 : z == 1 ? Z1 : z == 2 ? Z2 : Z3; }
-    __host__ __device__ static constexpr int maxbit() {
-        int mz = 1;
-        for (int z = 0; z < NZ_; ++z) mz = zeta(z) > mz ? zeta(z) : mz;
-        int b = 0;
-        while ((1 << (b + 1)) <= mz) ++b;
-        return b;
-    }
-};
-
+// ---------------------------------------------------------------- powers
 // X^E from the square chain ch[b] = X^(2^b); E is a compile-time constant
 // after unrolling, so the bit tests fold away.
 template <int E, typename T>
@@ -539,328 +688,348 @@ __device__ __forceinline__ void powers2(const DevModel& m, float2 X, float2 (&Tz
     }
 }
 
-template <class S>
-__device__ __forceinline__ int n_eta(const DevModel& m) {
-    return S::kFixed ? S::NE : m.fe;
-}
 
 // ---------------------------------------------------------------- pass 1
-template <typename T, class S>
-__global__ void __launch_bounds__(32 * kWarps, sizeof(T) == 4 ? 7 : 4) k_sfv_fast(Batch b, DevModel m, int mm, int mlo, int last) {
-    constexpr int NL = S::NL, NZ = S::NZ, NE = S::NE, P = S::P;
+// One k-step (4 pairs) of the FP64 tensor cores (mma.sync m8n8k4, thread t:
+// A[t/4][t%4], B[t%4][t/4], C[t/4][2 (t%4) + v]).
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double bb) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(bb));
+}
+
+// candidate-test vector of a slot: the FP32 copy (FP64 form) or the FP32
+// relative vector itself
+__device__ __forceinline__ void cvec(const FSmem<double>& s, int k, float& x, float& y, float& z) {
+    const float4 v = s.sp[k];
+    x = v.x;
+    y = v.y;
+    z = v.z;
+}
+__device__ __forceinline__ void cvec(const FSmem<float>& s, int k, float& x, float& y, float& z) {
+    const V4<float> v = s.nb[k];
+    x = v.x;
+    y = v.y;
+    z = v.z;
+}
+
+// Bits of word w (slots 32 w ..) that a row of rank ra may pair with: ranks
+// ra + d0 .. ra + d0 + nd - 1 whose block has functions.
+template <typename T>
+__device__ __forceinline__ unsigned allowed(const FSmem<T>& s, int nel, int ra, int d0, int nd, int w) {
+    unsigned m = 0;
+#pragma unroll 1
+    for (int rb = ra + d0; rb < nel && rb < ra + d0 + nd; ++rb) {
+        if (s.tm[ra * nel + rb] == 255) continue;
+        const int lo = max(s.rst[rb] - 32 * w, 0), hi = min(s.rst[rb + 1] - 32 * w, 32);
+        if (lo < hi) m |= (hi == 32 ? ~0u : (1u << hi) - 1u) & ~((1u << lo) - 1u);
+    }
+    return m;
+}
+
+// Bound by instruction issue.  The neighbours are staged by element, rarest
+// element first.  Contributing pairs (r_jk < rc) come row by row: for 32 rows
+// at a time, each neighbour in turn is tested against 32 others (a ballot per
+// row and word, 10 instructions for 32 candidates), the bits are counted and
+// each lane writes its row's pairs to its place in the list.  A chunk of 32
+// pairs, one per lane, is evaluated up to its powers
+// T[l, z] = (1 + lambda_l cos)^zeta_z and factors Y[e]; the sums over pairs
+//   acc[(l, z), (block, e)] += T[l, z] Y[e]
+// are a matrix product of the FP64 tensor cores over the chunk (8 k-steps of
+// 4 pairs): rows (l, z), columns (partner element of the row's element, e), a
+// pair's Y entering the columns of its own block.  So a chunk may hold pairs
+// of several blocks, the sums are spread over the lanes (2 per lane and tile,
+// no reduction across lanes) and G is written once per element of the rows.
+// The FP32 form feeds the same product (sums in FP64).
+template <typename T, class S, bool kB>
+__global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, DevModel m, int mm, int part) {
+    constexpr int NL = S::NL, NZ = S::NZ, NE = S::NE, P = S::P, A = kAx<S>;
+    // row tiles, blocks per accumulator tile, accumulator tiles
+    constexpr int MT = kTRows<S> / 8, SL = 8 / NE, GA = 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    FSmem<T> s = fcarve<T>(smem_raw + wib * fast_warp_bytes<T>(mm, m.g2max, m.nblk, P, false), mm, m.g2max,
-                           m.nblk, P, false);
-    const int nel = m.nel;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    FSmem<T> s = fcarve<T, S>(smem_raw + wib * fast_warp_bytes<T, S>(mm, m.nel, m.g2max, m.nblk, false), mm, m.nel, m.g2max, m.nblk, false);
+    const int nel = m.nel, nblk = m.nblk;
     T* Gout = Buf<T>::G(b);
     const int ne = n_eta<S>(m);
+    // fragment rows and columns of this lane
+    const T* ta = s.tb + (lane >> 2) * kTs + (lane & 3);
+    const T* ya = s.yb + (lane >> 2) * kTs + (lane & 3);
+    const int cap = list_cap(mm);
+    for (int q = lane; q < 8 * kTs; q += 32) s.yb[q] = (T)0;
+    __syncwarp();
     // work counters of this warp's atoms (profiling), added to b.stats once at the end
     unsigned long long st_ent = 0, st_cand = 0, st_pairs = 0, st_g2 = 0;
-    for (int i = blockIdx.x * kWarps + wib; i < b.natoms; i += gridDim.x * kWarps) {
+    const int total_atoms = part == kPartWide ? b.wide[0] : b.natoms;
+    for (int q = blockIdx.x * nw + wib; q < total_atoms; q += gridDim.x * nw) {
+        const int i = part == kPartWide ? b.wide[2 + q] : q;
         const int c = b.elem[i];
         if (c < 0) continue;
         const int M = b.nei_off[i + 1] - b.nei_off[i];
-        // this launch takes the atoms with mlo < M <= mm (see run_spec)
+        // more neighbours than this launch's shared memory takes: to the list
+        // of the launch that follows (see run_form)
         if (M > mm) {
-            if (last && lane == 0) atomicOr(&b.status[0], 4);
+            if (lane == 0) {
+                if (part == kPartFirst) b.wide[2 + atomicAdd(&b.wide[0], 1)] = i;
+                else atomicOr(&b.status[0], 4);
+            }
             continue;
         }
-        if (M <= mlo) continue;
-        const int Ms = fstage<T, false>(b, m, i, c, s, lane, M);
+        const int Ms = fstage<T, S, false, kB>(b, m, i, c, s, lane, M);
         const T rc = (T)m.rc[c], inv_rc = (T)(1.0 / m.rc[c]), rc2 = rc * rc;
         const double rc2d = m.rc[c] * m.rc[c];
+        // The FP64 form tests candidates on FP32 copies of the relative
+        // vectors.  Their rounding moves d^2 by less than 8e-7 rc^2 (vectors
+        // within rc, components to 2^-24), so with this margin no pair within
+        // rc is missed; one let in beyond rc has u = 0 and adds zeros.
+        const float rc2s = sizeof(T) == 8 ? (float)rc2d * (1.0f + 2e-6f) : (float)rc2;
         T* Gi = Gout + (size_t)i * m.nsf_max;
         const double* mean = m.smean + (size_t)c * m.nsf_max;
         const double* iwidth = m.sinvw + (size_t)c * m.nsf_max;
 
-        // radial SFs: lane = SF, its neighbour element's staged neighbours in
-        // order.  (A lane per (neighbour, SF) with shuffle sums was measured
-        // slower in both precisions: 25.4 against 20.8 ms per C4 step in
-        // FP64, 14.9 against 12.8 in FP32.  Groups of lanes per neighbour
-        // element, each lane a function and a share of the neighbours, with a
-        // butterfly over the groups, gained nothing.)
-        const int r0 = m.g2_off[c * nel], r1 = m.g2_off[c * nel + nel];
-        for (int f = r0 + lane; f < r1; f += 32) {
-            const SF2 q = m.g2[f];
-            const T eta = (T)q.eta, rs = (T)q.rs;
-            T acc = (T)0;
-            for (int t = s.est[q.nel]; t < s.est[q.nel + 1]; ++t) {
-                const T x = s.nb[t].w - rs;
-                acc += xexp(-eta * x * x) * s.ax[t].x;
-            }
-            Gi[q.sf] = (T)(((double)acc - mean[q.sf]) * iwidth[q.sf]);
-        }
-
-        unsigned long long n_cand = 0, n_pairs = 0;
-        // Contributing pairs of all element-pair blocks go through one queue
-        // (entries j | k << 10 | block << 20, enumeration order), so a chunk of
-        // 32 pairs may hold the end of one block and the start of the next:
-        // the lanes of the older block add their terms, every lane writes its
-        // sums of that block for the reduction (the newer block's lanes the
-        // sums they held before this chunk), and then the newer block's lanes
-        // start their sums with their terms.  The queue holds at most two
-        // blocks, and a block's remainder is carried into the next block's
-        // chunks instead of being flushed as a partly filled chunk.
-        // FP32 with two lambdas: the accumulators packed over lambda,
-        // acc2[z * NE + e] = (acc[0, z, e], acc[1, z, e]).  FP64 with two
-        // lambdas: the lambdas split over a lane pair (lane, lane ^ 1), each
-        // lane adding lambda_(lane & 1) of both pairs' terms, acc[z * NE + e]
-        // (half the accumulators and half the reduction per lane).
-        constexpr bool kPk = sizeof(T) == 4 && NL == 2;
-        constexpr bool kSp = sizeof(T) == 8 && NL == 2;
-        constexpr int NA = kSp ? P / 2 : P;
-        T acc[NA];
-        float2 acc2[kPk ? NZ * NE : 1];
-        auto zero_acc = [&]() {
-#pragma unroll
-            for (int p = 0; p < NA; ++p) acc[p] = (T)0;
-#pragma unroll
-            for (int p = 0; p < (kPk ? NZ * NE : 1); ++p) acc2[p] = f2(0.0f);
-        };
-        // terms of one pair: cos(theta) and Y[e] = exp(-eta_e R) fc_ij fc_ik fc_jk
-        auto pair_terms = [&](unsigned pk, T& cth, T (&Y)[NE]) {
-            const int pj = pk & 0x3ff, pq = (pk >> 10) & 0x3ff;
-            const V4<T> a = s.nb[pj], bq = s.nb[pq];
-            const V4<T> xa = s.ax[pj], xb = s.ax[pq];
-            const T cx = bq.x - a.x, cy = bq.y - a.y, cz = bq.z - a.z;
-            const T rjk2 = cx * cx + cy * cy + cz * cz;
-            const T rjk = xsqrt(rjk2);
-            const T tj = xtanh(pair_u(s, pj, pq, rc2d, rc, inv_rc, rjk));
-            const T fjk = tj * tj * tj;
-            const T t1 = -xa.z * xb.z;  // -1/(rj rk)
-            cth = (T)0.5 * (rjk2 - a.w * a.w - bq.w * bq.w) * t1;
-            const T fcp = xa.x * xb.x * fjk;
-            const T R = a.w * a.w + bq.w * bq.w + rjk2;
-            eta_exps<NE, false>(m, ne, R, Y);
-#pragma unroll
-            for (int e = 0; e < NE; ++e) Y[e] *= fcp;
-        };
-        // acc[l, z, e] += (1 + lambda_l cos)^zeta_z Y[e]
-        auto accumulate = [&](T cth, const T (&Y)[NE]) {
-            if constexpr (kPk) {
-                const float2 X = __ffma2_rn(make_float2((float)m.lam[0], (float)m.lam[1]), f2((float)cth), f2(1.0f));
-                float2 Tz[NZ], Tp[NZ];
-                powers2<S, false>(m, X, Tz, Tp);
-#pragma unroll
-                for (int z = 0; z < NZ; ++z)
-#pragma unroll
-                    for (int e = 0; e < NE; ++e) acc2[z * NE + e] = __ffma2_rn(Tz[z], f2((float)Y[e]), acc2[z * NE + e]);
-            } else if constexpr (kSp) {
-                const T lam = (lane & 1) ? (T)m.lam[1] : (T)m.lam[0];
-                T Tz[NZ], Tp[NZ];
-                powers<S, false>(m, (T)1 + lam * cth, Tz, Tp);
-#pragma unroll
-                for (int z = 0; z < NZ; ++z)
-#pragma unroll
-                    for (int e = 0; e < NE; ++e) acc[z * NE + e] += Tz[z] * Y[e];
-            } else {
-#pragma unroll
-                for (int l = 0; l < NL; ++l) {
-                    T Tz[NZ], Tp[NZ];
-                    powers<S, false>(m, (T)1 + (T)m.lam[l] * cth, Tz, Tp);
-#pragma unroll
-                    for (int z = 0; z < NZ; ++z)
-#pragma unroll
-                        for (int e = 0; e < NE; ++e) acc[(l * NZ + z) * NE + e] += Tz[z] * Y[e];
-                }
-            }
-        };
-        // every lane's sums of block t -> G of block t (warp reduction through
-        // shared memory: rows of P + 1, or of P/2 + 1 with the lambda split);
-        // called by all lanes
-        auto emit = [&](int t) {
-            if constexpr (kSp) {
-                // rows of P/2: lane L holds lambda_(L & 1); output p = (l, z, e)
-                // sums the 16 rows of parity l, 32/P helper lanes per output
-                T* row = s.red + lane * (P / 2 + 1);
-#pragma unroll
-                for (int q = 0; q < P / 2; ++q) row[q] = acc[q];
-                __syncwarp();
-                constexpr int NH = 32 / P > 0 ? 32 / P : 1;
-                static_assert(16 % NH == 0, "helpers per output");
-                const int p = lane % P, hh = lane / P;
-                const int l = p / (NZ * NE), q = p % (NZ * NE);
-                T sum = (T)0;
-                if (hh < NH)
-#pragma unroll
-                    for (int r = 0; r < 16 / NH; ++r) sum += s.red[(2 * (hh + r * NH) + l) * (P / 2 + 1) + q];
-#pragma unroll
-                for (int off = P; off < 32; off <<= 1) sum += __shfl_xor_sync(kFull, sum, off);
-                __syncwarp();
-                if (lane < P) {
-                    const int sf = m.pmap[((size_t)c * m.nblk + t) * P + lane];
-                    if (sf >= 0) {
-                        const int z = (lane / NE) % NZ;
-                        Gi[sf] = (T)(((double)((T)m.pfz[z] * sum) - mean[sf]) * iwidth[sf]);
+        // radial SFs: lane = neighbour, its element's functions eight at a time
+        // (rows); the sums over neighbours are products with fc in the column
+        // of the neighbour's rank
+        for (int fb = 0; fb < m.g2el_max; fb += 8)
+            for (int x0 = 0; x0 < nel; x0 += 8) {
+                double racc[2] = {0.0, 0.0};
+                for (int t0 = 0; t0 < Ms; t0 += 32) {
+                    const int t = t0 + lane;
+                    const bool live = t < Ms;
+                    const int rank = live ? rank_of(s.ax[t * A + 1]) : 0;
+                    const int g = c * nel + s.ord[rank];
+                    const int f0 = m.g2_off[g] + fb, nf = live ? m.g2_off[g + 1] - f0 : 0;
+                    const T r = live ? s.rf[2 * t] : (T)0;
+                    const bool mine = live && rank >= x0 && rank < x0 + 8;
+                    if (mine) s.yb[(rank - x0) * kTs + lane] = s.rf[2 * t + 1];
+#pragma unroll 2
+                    for (int f = 0; f < 8; ++f) {
+                        T e = (T)0;
+                        if (f < nf) {
+                            const SF2 q = m.g2[f0 + f];
+                            const T x = r - (T)q.rs;
+                            e = rad_exp<kB>(-(T)q.eta * x * x);
+                        }
+                        s.tb[f * kTs + lane] = e;
                     }
+                    __syncwarp();
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks) dmma(racc, (double)ta[4 * ks], (double)ya[4 * ks]);
+                    __syncwarp();
+                    if (mine) s.yb[(rank - x0) * kTs + lane] = (T)0;
+                    __syncwarp();
                 }
-                return;
-            }
-            {
-                T* row = s.red + lane * (P + 1);
-                if constexpr (kPk) {
 #pragma unroll
-                    for (int q = 0; q < NZ * NE; ++q) {
-                        row[q] = (T)acc2[q].x;            // l = 0
-                        row[NZ * NE + q] = (T)acc2[q].y;  // l = 1
-                    }
-                } else {
-#pragma unroll
-                    for (int p = 0; p < P; ++p) row[p] = acc[p];
-                }
-            }
-            __syncwarp();
-            constexpr int NH = 32 / P > 0 ? 32 / P : 1;
-            const int p = lane % P, h = lane / P;
-            T sum = (T)0;
-            if (h < NH)
-#pragma unroll
-                for (int r = 0; r < 32 / NH; ++r) sum += s.red[(h + r * NH) * (P + 1) + p];
-#pragma unroll
-            for (int off = P; off < 32; off <<= 1) sum += __shfl_xor_sync(kFull, sum, off);
-            __syncwarp();
-            if (lane < P) {
-                const int sf = m.pmap[((size_t)c * m.nblk + t) * P + lane];
-                if (sf >= 0) {
-                    const int z = (lane / NE) % NZ;
-                    Gi[sf] = (T)(((double)((T)m.pfz[z] * sum) - mean[sf]) * iwidth[sf]);
-                }
-            }
-        };
-        int qlen = 0;   // pending queue entries
-        int cur = -1;   // block whose sums the accumulators hold
-        zero_acc();
-        // process the first n queue entries (all lanes call)
-        auto flush = [&](int n) {
-            const unsigned pk = lane < n ? s.queue[lane] : 0u;
-            const int tg = lane < n ? (int)(pk >> 20) : cur;
-            T cth = (T)0, Y[NE];
-#pragma unroll
-            for (int e = 0; e < NE; ++e) Y[e] = (T)0;
-            if (lane < n) pair_terms(pk, cth, Y);
-            // a chunk that ends block cur and starts the next one (the last
-            // lane's): cur's lanes add their terms, cur is reduced, then the
-            // next block's lanes start their sums
-            const bool straddle = __any_sync(kFull, tg != cur);
-            const int nxt = straddle ? __shfl_sync(kFull, tg, n - 1) : cur;
-            if constexpr (sizeof(T) == 8) {
-                // FP64: one call site of the accumulation, in two passes
-                // around the reduction (smaller code: the value pass was
-                // instruction-fetch bound; 24.7 against 25.4 ms on the C4
-                // batch).  With the lambda split this lane also takes its
-                // partner's (lane ^ 1) pair, whose terms come by shuffle.
-                T cth_o = (T)0, Y_o[NE];
-                int tg_o = cur;
-                const bool live_o = kSp && (lane ^ 1) < n;
-                if constexpr (kSp) {
-                    cth_o = __shfl_xor_sync(kFull, cth, 1);
-#pragma unroll
-                    for (int e = 0; e < NE; ++e) Y_o[e] = __shfl_xor_sync(kFull, Y[e], 1);
-                    tg_o = __shfl_xor_sync(kFull, tg, 1);
-                }
-                for (int pass = 0; pass < (straddle ? 2 : 1); ++pass) {
-                    if (pass == 1) {
-                        emit(cur);
-                        zero_acc();
-                        cur = nxt;
-                    }
-                    for (int w2 = 0; w2 < (kSp ? 2 : 1); ++w2) {
-                        const bool own = w2 == 0;
-                        if (own ? (lane < n && tg == cur) : (live_o && tg_o == cur)) {
-                            T Yw[NE];
-#pragma unroll
-                            for (int e = 0; e < NE; ++e) Yw[e] = own ? Y[e] : Y_o[e];
-                            accumulate(own ? cth : cth_o, Yw);
+                for (int v = 0; v < 2; ++v) {
+                    const int rank = x0 + 2 * (lane & 3) + v;
+                    if (rank < nel) {
+                        const int g = c * nel + s.ord[rank], f = m.g2_off[g] + fb + (lane >> 2);
+                        if (f < m.g2_off[g + 1]) {
+                            const int sf = m.g2[f].sf;
+                            Gi[sf] = (T)((racc[v] - mean[sf]) * iwidth[sf]);
                         }
                     }
                 }
-            } else if (!straddle) {
-                // FP32 at 72 registers: the two-pass loop spills (70.4 against 73.0 ms)
-                if (lane < n) accumulate(cth, Y);
-            } else {
-                if (lane < n && tg == cur) accumulate(cth, Y);
-                emit(cur);
-                zero_acc();
-                if (lane < n && tg == nxt) accumulate(cth, Y);
-                cur = nxt;
+            }
+
+        if constexpr (sizeof(T) == 8) {
+            // the radial distances give way to the candidate test's vectors
+            for (int t = lane; t < Ms; t += 32) {
+                const V4<T> d = s.nb[t];
+                s.sp[t] = make_float4((float)d.x, (float)d.y, (float)d.z, 0.0f);
             }
             __syncwarp();
-            const int rem = qlen - n;
-            unsigned v = 0;
-            if (lane < rem) v = s.queue[n + lane];
-            __syncwarp();
-            if (lane < rem) s.queue[lane] = v;
-            __syncwarp();
-            qlen = rem;
-        };
-        for (int t = 0; t < m.nblk; ++t) {
-            const int gb = m.g4_off[c * m.nblk + t], ge = m.g4_off[c * m.nblk + t + 1];
-            if (ge == gb) continue;
-            if (cur < 0) cur = t;
-            const int ea = m.blk_a[t], eb = m.blk_b[t];
-            const int sa = s.est[ea], na = s.est[ea + 1] - sa;
-            const int sb = s.est[eb], nb = s.est[eb + 1] - sb;
-            const bool same = (ea == eb);
-            const int ncand = same ? na * (na - 1) / 2 : na * nb;
-            const float inv_nb = nb > 0 ? 1.0f / (float)nb : 0.0f;
-            n_cand += ncand;
-            for (int cb = 0; cb < ncand; cb += 32) {
-                const int cidx = cb + lane;
-                bool ok = cidx < ncand;
-                int j = 0, k = 0;
-                if (ok) {
-                    fpair(cidx, sa, na, sb, nb, same, inv_nb, j, k);
-                    const V4<T> a = s.nb[j], bb = s.nb[k];
-                    const T ex = bb.x - a.x, ey = bb.y - a.y, ez = bb.z - a.z;
-                    ok = ex * ex + ey * ey + ez * ez < rc2;
+        }
+
+        int n_pairs = 0;
+        double acc[GA][MT][2];
+#pragma unroll
+        for (int g = 0; g < GA; ++g)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) acc[g][mt][0] = acc[g][mt][1] = 0.0;
+        // potentials with more elements than the accumulators hold blocks for:
+        // several passes over the rows, each with the partners of one range of
+        // ranks
+        for (int d0 = 0; d0 < nel; d0 += GA * SL) {
+            int cur = 0;  // rank whose blocks the accumulators hold
+            int qn = 0;  // listed pairs
+            for (int j0 = 0; j0 < Ms || j0 == 0; j0 += 32) {
+                // rows j0 .. j0 + 31: lane = row, the bits of its partners k > j
+                const int nrow = min(32, Ms - j0);
+                int cnt = 0;
+                for (int w = j0 >> 5; 32 * w < Ms; ++w) {
+                    const int k = 32 * w + lane;
+                    float kx = 1e18f, ky = 0.0f, kz = 0.0f;
+                    if (k < Ms) cvec(s, k, kx, ky, kz);
+                    unsigned mw = 0;
+                    for (int jj = 0; jj < nrow; jj += 4)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            float jx, jy, jz;
+                            cvec(s, j0 + jj + u, jx, jy, jz);
+                            const float ex = kx - jx, ey = ky - jy, ez = kz - jz;
+                            const unsigned bal = __ballot_sync(kFull, ex * ex + ey * ey + ez * ez < rc2s);
+                            mw = lane == jj + u ? bal : mw;
+                        }
+                    if (32 * w == j0) mw &= ~((2u << lane) - 1u);
+                    if (lane >= nrow) mw = 0;
+                    if (!m.g4_full || nel > GA * SL) mw &= lane < nrow ? allowed(s, nel, rank_of(s.ax[(j0 + lane) * A + 1]), d0, GA * SL, w) : 0u;
+                    s.mask[32 * w + lane] = mw;
+                    cnt += __popc(mw);
                 }
-                const unsigned bal = __ballot_sync(kFull, ok);
-                const unsigned ent = (unsigned)j | ((unsigned)k << 10) | ((unsigned)t << 20);
-                if (ok) s.queue[qlen + __popc(bal & lanemask_lt())] = ent;
-                if (ok && b.pairs) {
-                    // contributing-pair list for the gradient pass (enumeration order)
-                    const long long slot = (long long)n_pairs + __popc(bal & lanemask_lt());
-                    if (slot < b.pcap) b.pairs[(size_t)i * b.pcap + slot] = ent;
+                int incl = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += v;
                 }
-                qlen += __popc(bal);
-                n_pairs += __popc(bal);
-                __syncwarp();
-                while (qlen >= 32) flush(32);
-            }
-            // block t is screened.  An older block still pending in the queue
-            // (its remainder followed by t's pairs, fewer than 32 together) is
-            // finished now, and then t with it.
-            if (cur != t) {
-                if (qlen > 0) flush(qlen);
-                if (cur != t) {  // t had no contributing pairs
-                    emit(cur);
-                    zero_acc();
-                    cur = t;
-                }
-                if (qlen > 0) flush(qlen);
-                emit(t);
-                zero_acc();
-                cur = -1;
-            } else if (qlen == 0) {
-                emit(t);
-                zero_acc();
-                cur = -1;
+                const int off = incl - cnt, total = __shfl_sync(kFull, incl, 31);
+                int start = 0;
+                bool more;
+                do {
+                    // the rows that fit into the list, in order
+                    const bool fits = off >= start && incl - start <= cap - qn;
+                    const unsigned who = __ballot_sync(kFull, fits);
+                    if (fits && cnt > 0) {
+                        unsigned* dst = s.queue + qn + off - start;
+                        for (int w = j0 >> 5; 32 * w < Ms; ++w) {
+                            unsigned mw = s.mask[32 * w + lane];
+                            const unsigned row = (unsigned)(j0 + lane) | ((unsigned)(32 * w) << 10);
+                            while (mw) {
+                                *dst++ = row + ((unsigned)(__ffs(mw) - 1) << 10);
+                                mw &= mw - 1;
+                            }
+                        }
+                    }
+                    const int end = __shfl_sync(kFull, incl, 31 - __clz(who));
+                    qn += end - start;
+                    start = end;
+                    more = start < total;
+                    const bool fin = !more && j0 + 32 >= Ms;
+                    __syncwarp();
+                    int pos = 0;
+                    // (the last one of a pass also when it is empty: it writes
+                    // the sums of the ranks that are left)
+                    while (qn - pos >= 32 || (fin && cur < nel)) {
+                        // a chunk of 32 pairs, one per lane
+                        const int n = min(32, qn - pos);
+                        int rj = -1, dr = 0;
+                        T cth = (T)0, Y[NE];
+#pragma unroll
+                        for (int e = 0; e < NE; ++e) Y[e] = (T)0;
+                        if (lane < n) {
+                            const unsigned pk = s.queue[pos + lane];
+                            const int pj = pk & 0x3ff, pq = pk >> 10;
+                            const V4<T> a = s.nb[pj], bq = s.nb[pq];
+                            T xa[A], xb[A];
+                            ldax<A>(s.ax, pj, xa);
+                            ldax<A>(s.ax, pq, xb);
+                            rj = rank_of(xa[1]);
+                            const int rq = rank_of(xb[1]);
+                            dr = rq - rj - d0;
+                            // contributing-pair list for the gradient pass
+                            if (b.pairs && n_pairs + lane < b.pcap)
+                                b.pairs[(size_t)i * b.pcap + n_pairs + lane] = pk | ((unsigned)s.tm[rj * nel + rq] << 20);
+                            const T cx = bq.x - a.x, cy = bq.y - a.y, cz = bq.z - a.z;
+                            const T rjk2 = cx * cx + cy * cy + cz * cz;
+                            T E[NE];
+                            eta_exps<NE, kB>(m, ne, rjk2, E);
+                            const T tj = xtanh(pair_u(s, pj, pq, rc2d, rc, inv_rc, xsqrt(rjk2)));
+                            const T fjk = tj * tj * tj;
+                            cth = (T)0.5 * (a.w + bq.w - rjk2) * (xa[0] * xb[0]);
+#pragma unroll
+                            for (int e = 0; e < NE; ++e) Y[e] = xa[2 + e] * xb[2 + e] * (E[e] * fjk);
+                        }
+                        if constexpr (sizeof(T) == 4 && NL == 2) {
+                            const float2 X = __ffma2_rn(make_float2((float)m.lam[0], (float)m.lam[1]), f2((float)cth), f2(1.0f));
+                            float2 Tz[NZ], Tp[NZ];
+                            powers2<S, false>(m, X, Tz, Tp);
+#pragma unroll
+                            for (int z = 0; z < NZ; ++z) {
+                                s.tb[z * kTs + lane] = Tz[z].x;
+                                s.tb[(NZ + z) * kTs + lane] = Tz[z].y;
+                            }
+                        } else {
+#pragma unroll
+                            for (int l = 0; l < NL; ++l) {
+                                T Tz[NZ], Tp[NZ];
+                                powers<S, false>(m, (T)1 + (T)m.lam[l] * cth, Tz, Tp);
+#pragma unroll
+                                for (int z = 0; z < NZ; ++z) s.tb[(l * NZ + z) * kTs + lane] = Tz[z];
+                            }
+                        }
+                        __syncwarp();
+                        const int rlast = fin && pos + n == qn ? nel : __shfl_sync(kFull, rj, n - 1);
+                        for (;;) {
+#pragma unroll
+                            for (int g = 0; g < GA; ++g) {
+                                // the pairs of these blocks put their factors into
+                                // the columns of their block
+                                const bool in = rj == cur && dr >= g * SL && dr < (g + 1) * SL;
+                                if (!__any_sync(kFull, in)) continue;
+                                T* yc = s.yb + (dr - g * SL) * NE * kTs + lane;
+                                if (in)
+#pragma unroll
+                                    for (int e = 0; e < NE; ++e) yc[e * kTs] = Y[e];
+                                __syncwarp();
+#pragma unroll
+                                for (int ks = 0; ks < 8; ++ks)
+#pragma unroll
+                                    for (int mt = 0; mt < MT; ++mt) dmma(acc[g][mt], (double)ta[mt * 8 * kTs + 4 * ks], (double)ya[4 * ks]);
+                                __syncwarp();
+                                if (in)
+#pragma unroll
+                                    for (int e = 0; e < NE; ++e) yc[e * kTs] = (T)0;
+                                __syncwarp();
+                            }
+                            if (rlast == cur) break;
+                            // rank cur is complete: its sums -> G
+#pragma unroll
+                            for (int g = 0; g < GA; ++g) {
+                                if (cur + d0 + g * SL >= nel) break;  // uniform
+#pragma unroll
+                                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                                    for (int v = 0; v < 2; ++v) {
+                                        const int row = mt * 8 + (lane >> 2), col = 2 * (lane & 3) + v;
+                                        const int rb = cur + d0 + g * SL + col / NE;
+                                        const int t = row < NL * NZ && rb < nel ? s.tm[cur * nel + rb] : 255;
+                                        if (t < 255) {
+                                            const size_t at = ((size_t)c * nblk + t) * P + row * NE + col % NE;
+                                            const int sf = m.pmap[at];
+                                            const double2 q = m.pscale[at];
+                                            if (sf >= 0) Gi[sf] = (T)fma(q.x, acc[g][mt][v], q.y);
+                                        }
+                                        acc[g][mt][v] = 0.0;
+                                    }
+                            }
+                            if (++cur == nel) break;
+                        }
+                        __syncwarp();
+                        pos += n;
+                        n_pairs += n;
+                    }
+                    // the remainder moves to the front
+                    const unsigned v = pos + lane < qn ? s.queue[pos + lane] : 0u;
+                    __syncwarp();
+                    s.queue[lane] = v;
+                    qn -= pos;
+                    __syncwarp();
+                } while (more);
             }
         }
-        if (cur >= 0) {
-            if (qlen > 0) flush(qlen);
-            emit(cur);
-            zero_acc();
-        }
-        if (b.pairs && lane == 0) b.npairs[i] = n_pairs > (unsigned long long)INT32_MAX ? INT32_MAX : (int)n_pairs;
+        if (b.pairs && lane == 0) b.npairs[i] = n_pairs;
         if (b.stats) {
             // radial terms: staged neighbours of each element x the centre's radial SFs for it
             for (int el = 0; el < nel; ++el)
-                st_g2 += (unsigned long long)(s.est[el + 1] - s.est[el]) *
+                st_g2 += (unsigned long long)s.cnt[el] *
                          (unsigned long long)(m.g2_off[c * nel + el + 1] - m.g2_off[c * nel + el]);
+            for (int t = 0; t < nblk; ++t)
+                if (m.g4_off[c * nblk + t + 1] > m.g4_off[c * nblk + t]) {
+                    const int na = s.cnt[m.blk_a[t]], nb = s.cnt[m.blk_b[t]];
+                    st_cand += m.blk_a[t] == m.blk_b[t] ? na * (na - 1) / 2 : na * nb;
+                }
             st_ent += (unsigned long long)M;
-            st_cand += n_cand;
             st_pairs += n_pairs;
         }
         __syncwarp();
@@ -875,49 +1044,20 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(T) == 4 ? 7 : 4) k_sfv_fas
 }
 
 // ---------------------------------------------------------------- pass 2
-// (x, y, z) of every lane with `live` set added to gradient slot `slot`.  The
-// lanes naming one slot form a group (__match_any_sync); its lowest lane adds
-// the other members' values in ascending lane order (indexed shuffles, as many
-// rounds as the largest group has members) and writes the slot with one plain
-// read-modify-write, so no two lanes write one slot and the result does not
-// depend on timing.  (Shared-memory FP64 atomicAdd measured 5.6 ms of the 21 ms
-// FP64 gradient pass on the 4096-structure batch, against 0.3 ms for plain
-// read-modify-writes; rounds of an integer atomicMin that elect one lane per
-// slot cost as much as the atomics.)  Called by all lanes.
-template <typename T>
-__device__ __forceinline__ void group_add(const FSmem<T>& s, bool live, int slot, T x, T y, T z, int lane) {
-    const unsigned grp = __match_any_sync(kFull, live ? slot : -1 - lane);
-    const int most = __reduce_max_sync(kFull, __popc(grp));
-    const bool lead = live && (grp & lanemask_lt()) == 0;
-    unsigned rest = grp & ~(1u << lane);
-    T sx = x, sy = y, sz = z;
-    for (int r = 1; r < most; ++r) {
-        const int src = rest ? __ffs(rest) - 1 : lane;
-        const T ox = __shfl_sync(kFull, x, src);
-        const T oy = __shfl_sync(kFull, y, src);
-        const T oz = __shfl_sync(kFull, z, src);
-        if (rest) {
-            rest &= rest - 1;
-            sx += ox;
-            sy += oy;
-            sz += oz;
-        }
-    }
-    if (lead) {
-        s.gx[slot] += sx;
-        s.gy[slot] += sy;
-        s.gz[slot] += sz;
-    }
-}
-
 // Gradient contributions of up to 32 contributing pairs (one per lane; pk =
-// j | k << 10 | block << 20, live for lane < n): dE/dr_k added to slot k,
-// dE/dr_j summed over runs of equal j (lanes hold pairs in enumeration order,
-// so equal j are contiguous) and added once per run.  Called by all lanes.
-template <typename T, class S>
+// j | k << 10 | block << 20, live for lane < n).  Runs of equal j are
+// contiguous lanes with distinct k, so within a run dE/dr_k needs no care for
+// conflicts; dE/dr_j is summed over the run.  Each group of 32 / kCopies lanes
+// has accumulators of its own, so runs are cut at the groups' borders, the
+// groups work side by side, and a group with several runs takes them one
+// after the other: no two lanes ever update one value at a time, and the
+// sums do not depend on timing.  (Shared-memory FP64 atomics measured 5.6 of
+// the 21 ms FP64 gradient pass on the 4096-structure batch.)  Called by all
+// lanes.
+template <typename T, class S, bool kB>
 __device__ __forceinline__ void grad_pairs(const FSmem<T>& s, const DevModel& m, int ne, T rc, T inv_rc, double rc2d,
                                            unsigned pk_in, int n, int lane) {
-    constexpr int NL = S::NL, NZ = S::NZ, NE = S::NE, P = S::P;
+    constexpr int NL = S::NL, NZ = S::NZ, NE = S::NE, P = S::P, A = kAx<S>;
         // dE/dr_j of this lane's pair (summed over runs of equal j below) and
         // dE/dr_k
         int pj = -1 - lane, pq = -1 - lane;
@@ -928,36 +1068,36 @@ __device__ __forceinline__ void grad_pairs(const FSmem<T>& s, const DevModel& m,
             pq = (pk >> 10) & 0x3ff;
             const int pt = pk >> 20;
             const V4<T> a = s.nb[pj], bq = s.nb[pq];
-            const V4<T> xa = s.ax[pj], xb = s.ax[pq];
-            const T fj = xa.x, fk = xb.x, dfj = xa.y, dfk = xb.y;
+            T xa[A], xb[A];
+            ldax<A>(s.ax, pj, xa);
+            ldax<A>(s.ax, pq, xb);
             const T cx = bq.x - a.x, cy = bq.y - a.y, cz = bq.z - a.z;  // djk = r_j - r_k
             const T rjk2 = cx * cx + cy * cy + cz * cz;
+            T E[NE];
+            eta_exps<NE, kB>(m, ne, rjk2, E);
             T rjk, irjk;
             dist_inv(rjk2, rjk, irjk);
             const T tj = xtanh(pair_u(s, pj, pq, rc2d, rc, inv_rc, rjk)), tt = tj * tj;
             const T fjk = tt * tj;
-            const T dfjk = (T)(-3) * inv_rc * irjk * (tt - tt * tt);
-            const T irj = xa.z, irk = xb.z;
-            const T t1 = -irj * irk;
-            const T cth = (T)0.5 * (rjk2 - a.w * a.w - bq.w * bq.w) * t1;
-            const T dot = a.x * bq.x + a.y * bq.y + a.z * bq.z;
-            const T cj = dot * irj * irj * irj * irk, ck = dot * irk * irk * irk * irj;
-            const T fcp = fj * fk * fjk;
-            const T R = a.w * a.w + bq.w * bq.w + rjk2;
-            T Y[NE];
-            eta_exps<NE, true>(m, ne, R, Y);
+            const T dfjk = (T)(-3) * inv_rc * irjk * (tt - tt * tt);  // 2 d fc / d(r_jk^2)
+            const T h = xa[0] * xb[0];  // 1 / (r_ij r_ik)
+            const T cth = (T)0.5 * (a.w + bq.w - rjk2) * h;
             T SA[NE], SC[NE];
 #pragma unroll
             for (int e = 0; e < NE; ++e) SA[e] = SC[e] = (T)0;
-            T wa[P], wc[P];
-            ldvec<P>(s.WA + pt * P, wa);
-            ldvec<P>(s.WC + pt * P, wc);
+            // weights of the block; those of d/d cos are lambda zeta times
+            // them, and the factor goes to the powers (shared by the etas)
+            T wa[P];
+            ldvec<P>(s.WA + pt * kWp<S>, wa);
             if constexpr (sizeof(T) == 4 && NL == 2) {
                 // packed over lambda: the weights are staged as (l = 0, l = 1)
                 // pairs, wa[2 (z NE + e) + l] (see the staging in k_sfg_fast)
                 const float2 X = __ffma2_rn(make_float2((float)m.lam[0], (float)m.lam[1]), f2((float)cth), f2(1.0f));
                 float2 Tz[NZ], Tp[NZ];
                 powers2<S, true>(m, X, Tz, Tp);
+                const float2 lam = make_float2((float)m.lam[0], (float)m.lam[1]);
+#pragma unroll
+                for (int z = 0; z < NZ; ++z) Tp[z] = __fmul2_rn(Tp[z], __fmul2_rn(lam, f2((float)zeta_of<S>(m, z))));
                 float2 SA2[NE], SC2[NE];
 #pragma unroll
                 for (int e = 0; e < NE; ++e) SA2[e] = SC2[e] = f2(0.0f);
@@ -967,7 +1107,7 @@ __device__ __forceinline__ void grad_pairs(const FSmem<T>& s, const DevModel& m,
                     for (int e = 0; e < NE; ++e) {
                         const int q = 2 * (z * NE + e);
                         SA2[e] = __ffma2_rn(make_float2(wa[q], wa[q + 1]), Tz[z], SA2[e]);
-                        SC2[e] = __ffma2_rn(make_float2(wc[q], wc[q + 1]), Tp[z], SC2[e]);
+                        SC2[e] = __ffma2_rn(make_float2(wa[q], wa[q + 1]), Tp[z], SC2[e]);
                     }
 #pragma unroll
                 for (int e = 0; e < NE; ++e) {
@@ -980,48 +1120,54 @@ __device__ __forceinline__ void grad_pairs(const FSmem<T>& s, const DevModel& m,
                     T Tz[NZ], Tp[NZ];
                     powers<S, true>(m, (T)1 + (T)m.lam[l] * cth, Tz, Tp);
 #pragma unroll
+                    for (int z = 0; z < NZ; ++z) Tp[z] *= (T)m.lam[l] * zeta_of<S>(m, z);
+#pragma unroll
                     for (int z = 0; z < NZ; ++z)
 #pragma unroll
                         for (int e = 0; e < NE; ++e) {
                             SA[e] += wa[(l * NZ + z) * NE + e] * Tz[z];
-                            SC[e] += wc[(l * NZ + z) * NE + e] * Tp[z];
+                            SC[e] += wa[(l * NZ + z) * NE + e] * Tp[z];
                         }
                 }
             }
-            T A = (T)0, B = (T)0, C = (T)0;
+            // sums over the grid without fc_jk: value, eta-weighted value and
+            // d/d cos; then twice the derivatives of the pair's sum with
+            // respect to r_ij^2, r_ik^2 and r_jk^2
+            T V = (T)0, B = (T)0, C = (T)0;
 #pragma unroll
             for (int e = 0; e < NE; ++e) {
-                A += Y[e] * SA[e];
-                B += (T)m.eta4[e] * Y[e] * SA[e];
-                C += Y[e] * SC[e];
+                const T Y = xa[2 + e] * xb[2 + e] * E[e];
+                const T y = Y * SA[e];
+                V += y;
+                B += (T)m.eta4[e] * y;
+                C += Y * SC[e];
             }
-            const T B2 = (T)2 * B * fcp, Cf = C * fcp;
-            const T pj1 = A * fk * fj * dfjk, pj2 = A * fk * dfj * fjk;
-            const T pk1 = A * fj * fk * dfjk, pk2 = A * fj * dfk * fjk;
-            gjx = pj1 * cx - pj2 * a.x + B2 * (a.x - cx) + Cf * (t1 * bq.x + a.x * cj);
-            gjy = pj1 * cy - pj2 * a.y + B2 * (a.y - cy) + Cf * (t1 * bq.y + a.y * cj);
-            gjz = pj1 * cz - pj2 * a.z + B2 * (a.z - cz) + Cf * (t1 * bq.z + a.z * cj);
-            gkx = -pk1 * cx - pk2 * bq.x + B2 * (bq.x + cx) + Cf * (t1 * a.x + bq.x * ck);
-            gky = -pk1 * cy - pk2 * bq.y + B2 * (bq.y + cy) + Cf * (t1 * a.y + bq.y * ck);
-            gkz = -pk1 * cz - pk2 * bq.z + B2 * (bq.z + cz) + Cf * (t1 * a.z + bq.z * ck);
+            const T V2 = (T)2 * fjk * V, B2 = (T)2 * fjk * B, Cf = fjk * C;
+            const T q3 = dfjk * V - B2 - Cf * h;
+            const T q1 = V2 * xa[1] - B2 + Cf * (h - cth * xa[0] * xa[0]);
+            const T q2 = V2 * xb[1] - B2 + Cf * (h - cth * xb[0] * xb[0]);
+            gjx = q3 * cx - q1 * a.x;
+            gjy = q3 * cy - q1 * a.y;
+            gjz = q3 * cz - q1 * a.z;
+            gkx = -q3 * cx - q2 * bq.x;
+            gky = -q3 * cy - q2 * bq.y;
+            gkz = -q3 * cz - q2 * bq.z;
         }
-        group_add(s, lane < n, pq, gkx, gky, gkz, lane);
-        __syncwarp();
-        // Queue order is enumeration order, so pairs sharing j sit in
-        // contiguous lanes: a segmented suffix sum (fixed shuffle order)
-        // leaves each run's total in its first lane, which alone
-        // updates slot j -- instead of one conflicting atomic per lane.
+        constexpr int GL = 32 / kCopies;  // lanes of a group
+        const int prev_j = __shfl_up_sync(kFull, pj, 1);
+        const bool head = lane < n && ((lane & (GL - 1)) == 0 || prev_j != pj);
+        const unsigned heads = __ballot_sync(kFull, head);
+        const unsigned group = (kCopies == 1 ? kFull : (1u << (GL & 31)) - 1u) << (lane & ~(GL - 1));
+        const int run = __popc(heads & group & ~(~1u << lane)) - 1;   // this lane's run in its group
+        const int phases = __reduce_max_sync(kFull, __popc(heads & group));
         {
-            // every lane executes the shuffle (no short-circuit around it)
-            const int prev_j = __shfl_up_sync(kFull, pj, 1);
-            const bool head = lane == 0 || prev_j != pj;
-            const unsigned heads = __ballot_sync(kFull, head);
-            const unsigned after = heads & ~((2u << lane) - 1u);  // heads above this lane
-            const int last = after ? __ffs(after) - 2 : 31;        // last lane of my run
-            // doubling steps up to the longest run of the chunk (later steps
-            // would add nothing)
-            const int longest = __reduce_max_sync(kFull, head ? last - lane + 1 : 1);
-            for (int d = 1; d < longest; d <<= 1) {
+            // a segmented suffix sum over each run (fixed shuffle order)
+            // leaves dE/dr_j of the run in its first lane
+            const unsigned after = heads & group & (~1u << lane);  // heads above this lane
+            const int end = min(n, (lane | (GL - 1)) + 1);
+            const int last = after ? __ffs(after) - 2 : end - 1;   // last lane of my run
+#pragma unroll
+            for (int d = 1; d < GL; d <<= 1) {
                 const T ox = __shfl_down_sync(kFull, gjx, d);
                 const T oy = __shfl_down_sync(kFull, gjy, d);
                 const T oz = __shfl_down_sync(kFull, gjz, d);
@@ -1031,35 +1177,51 @@ __device__ __forceinline__ void grad_pairs(const FSmem<T>& s, const DevModel& m,
                     gjz += oz;
                 }
             }
-            // run totals into their slots (one block's runs name distinct
-            // slots; a chunk that spans two blocks can name one twice)
-            group_add(s, head && lane < n, pj, gjx, gjy, gjz, lane);
+        }
+        T* g = s.gx + (lane / GL) * 3 * s.gst;
+        for (int r = 0; r < phases; ++r) {
+            if (run == r && lane < n) {
+                g[pq] += gkx;
+                g[s.gst + pq] += gky;
+                g[2 * s.gst + pq] += gkz;
+                if (head) {
+                    g[pj] += gjx;
+                    g[s.gst + pj] += gjy;
+                    g[2 * s.gst + pj] += gjz;
+                }
+            }
+            __syncwarp();
         }
 }
 
-template <typename T, class S>
-// FP64: 5 blocks per SM at 96 registers (a few spills) beat 4 at 120 (23.1
-// against 23.9 ms on the C4 batch); the value pass loses at 5 (27.4 against 24.6)
-__global__ void __launch_bounds__(32 * kWarps, sizeof(T) == 4 ? 8 : 5) k_sfg_fast(Batch b, DevModel m, int mm, int mlo, int last) {
+template <typename T, class S, bool kB>
+// Bound by instruction issue and shared-memory latency: per pair two dozen
+// 16-byte shared loads, the geometry, cutoff, exponentials and powers again,
+// the contraction with dE/dG, and the update of two slots.
+__global__ void __launch_bounds__(32 * kWarps, kBlocksG<T>) k_sfg_fast(Batch b, DevModel m, int mm, int part) {
     constexpr int NL = S::NL, NZ = S::NZ, NE = S::NE, P = S::P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    FSmem<T> s = fcarve<T>(smem_raw + wib * fast_warp_bytes<T>(mm, m.g2max, m.nblk, P, true), mm, m.g2max,
-                           m.nblk, P, true);
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    FSmem<T> s = fcarve<T, S>(smem_raw + wib * fast_warp_bytes<T, S>(mm, m.nel, m.g2max, m.nblk, true), mm, m.nel, m.g2max, m.nblk, true);
     const int nel = m.nel;
     const T* dEdG = Buf<T>::dEdG(b);
     const int ne = n_eta<S>(m);
-    for (int i = blockIdx.x * kWarps + wib; i < b.natoms; i += gridDim.x * kWarps) {
+    const int total_atoms = part == kPartWide ? b.wide[1] : b.natoms;
+    for (int q = blockIdx.x * nw + wib; q < total_atoms; q += gridDim.x * nw) {
+        const int i = part == kPartWide ? b.wide[2 + q] : q;
         const int c = b.elem[i];
         if (c < 0) continue;
         const int M = b.nei_off[i + 1] - b.nei_off[i];
-        // this launch takes the atoms with mlo < M <= mm (see run_spec)
+        // more neighbours than this launch's shared memory takes: to the list
+        // of the launch that follows (see run_form)
         if (M > mm) {
-            if (last && lane == 0) atomicOr(&b.status[0], 4);
+            if (lane == 0) {
+                if (part == kPartFirst) b.wide[2 + atomicAdd(&b.wide[1], 1)] = i;
+                else atomicOr(&b.status[0], 4);
+            }
             continue;
         }
-        if (M <= mlo) continue;
-        const int Ms = fstage<T, true>(b, m, i, c, s, lane, M);
+        const int Ms = fstage<T, S, true, kB>(b, m, i, c, s, lane, M);
         const T rc = (T)m.rc[c], inv_rc = (T)(1.0 / m.rc[c]), rc2 = rc * rc;
         const double rc2d = m.rc[c] * m.rc[c];
         // w_s = dE/dG_s / width_s: radial SFs staged per slot of g2, angular
@@ -1074,35 +1236,33 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(T) == 4 ? 8 : 5) k_sfg_fas
         for (int q = lane; q < m.nblk * P; q += 32) {
             const int t = q / P, p = q % P;
             const int sf = m.pmap[((size_t)c * m.nblk + t) * P + p];
-            T wa = (T)0, wc = (T)0;
+            T wa = (T)0;
             const int l = p / (NZ * NE), z = (p / NE) % NZ;
-            if (sf >= 0) {
-                wa = (T)((double)dEdGi[sf] * iwc[sf]) * (T)m.pfz[z];
-                wc = wa * (T)m.lam[l] * (T)m.zet[z];
-            }
+            if (sf >= 0) wa = (T)((double)dEdGi[sf] * iwc[sf]) * (T)m.pfz[z];
             // FP32 with two lambdas: (l = 0, l = 1) pairs for the packed contraction
-            const int dst = (sizeof(T) == 4 && NL == 2) ? t * P + 2 * (p % (NZ * NE)) + l : q;
-            s.WA[dst] = wa;
-            s.WC[dst] = wc;
+            s.WA[t * kWp<S> + ((sizeof(T) == 4 && NL == 2) ? 2 * (p % (NZ * NE)) + l : p)] = wa;
         }
         __syncwarp();
 
         // radial: lane = neighbour slot
         for (int t = lane; t < Ms; t += 32) {
-            const int el = s.el[t];
+            const T r = s.gx[t], fc = s.gx[s.gst + t];
+            const int el = (int)s.gx[2 * s.gst + t];
             const int f0 = m.g2_off[c * nel + el], f1 = m.g2_off[c * nel + el + 1];
             const V4<T> d = s.nb[t];
-            const V4<T> x = s.ax[t];
+            const T ir = s.ax[t * kAx<S>], rho = s.ax[t * kAx<S> + 1];
             T coef = (T)0;
             for (int f = f0; f < f1; ++f) {
                 const SF2 q = m.g2[f];
-                const T eta = (T)q.eta, xr = d.w - (T)q.rs;
-                const T e = xexp(-eta * xr * xr);
-                coef += s.w2[f - r0] * (-e * x.y + (T)2 * eta * xr * x.z * e * x.x);
+                const T eta = (T)q.eta, xr = r - (T)q.rs;
+                coef += s.w2[f - r0] * rad_exp<kB>(-eta * xr * xr) * (eta * xr * ir - rho);
             }
-            s.gx[t] += coef * d.x;
-            s.gy[t] += coef * d.y;
-            s.gz[t] += coef * d.z;
+            coef *= (T)2 * fc;
+            s.gx[t] = coef * d.x;
+            s.gx[s.gst + t] = coef * d.y;
+            s.gx[2 * s.gst + t] = coef * d.z;
+#pragma unroll
+            for (int q = 3; q < 3 * kCopies; ++q) s.gx[q * s.gst + t] = (T)0;
         }
         __syncwarp();
 
@@ -1118,57 +1278,57 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(T) == 4 ? 8 : 5) k_sfg_fas
                 const int n = np - base < 32 ? np - base : 32;
                 const unsigned pk = nxt;
                 if (base + 32 < np) nxt = base + 32 + lane < np ? __ldg(pl + base + 32 + lane) : 0u;
-                grad_pairs<T, S>(s, m, ne, rc, inv_rc, rc2d, lane < n ? pk : 0u, n, lane);
+                grad_pairs<T, S, kB>(s, m, ne, rc, inv_rc, rc2d, lane < n ? pk : 0u, n, lane);
                 __syncwarp();
             }
         } else {
-        int qlen = 0;
-        for (int t = 0; t < m.nblk; ++t) {
-            const int gb = m.g4_off[c * m.nblk + t], ge = m.g4_off[c * m.nblk + t + 1];
-            const bool has = ge > gb;
-            const int ea = m.blk_a[t], eb = m.blk_b[t];
-            const int sa = s.est[ea], na = s.est[ea + 1] - sa;
-            const int sb = s.est[eb], nb = s.est[eb + 1] - sb;
-            const bool same = (ea == eb);
-            const int ncand = has ? (same ? na * (na - 1) / 2 : na * nb) : 0;
-            const float inv_nb = nb > 0 ? 1.0f / (float)nb : 0.0f;
-            const bool last_blk = (t == m.nblk - 1);
-            for (int cb = 0; cb < ncand || (last_blk && cb == 0); cb += 32) {
-                const int cidx = cb + lane;
-                bool ok = cidx < ncand;
-                int j = 0, k = 0;
-                if (ok) {
-                    fpair(cidx, sa, na, sb, nb, same, inv_nb, j, k);
-                    const V4<T> a = s.nb[j], bb = s.nb[k];
-                    const T ex = bb.x - a.x, ey = bb.y - a.y, ez = bb.z - a.z;
-                    ok = ex * ex + ey * ey + ez * ez < rc2;
+            unsigned qh = 0;
+            int qn = 0;
+            PairRows pr;
+            for (int t = 0; t <= m.nblk; ++t) {
+                const bool fin = t == m.nblk;
+                {
+                    const int ea = fin ? 0 : m.blk_a[t], eb = fin ? 0 : m.blk_b[t];
+                    const bool has = !fin && m.g4_off[c * m.nblk + t + 1] > m.g4_off[c * m.nblk + t];
+                    pr.start(s.est[ea], s.cnt[ea], s.est[eb], s.cnt[eb], ea == eb, has, lane);
                 }
-                const unsigned bal = __ballot_sync(kFull, ok);
-                if (ok) s.queue[qlen + __popc(bal & lanemask_lt())] = (unsigned)j | ((unsigned)k << 10) | ((unsigned)t << 20);
-                qlen += __popc(bal);
-                __syncwarp();
-                const bool flush_all = last_blk && cb + 32 >= ncand;
-                while (qlen >= 32 || (flush_all && qlen > 0)) {
-                    const int n = qlen < 32 ? qlen : 32;
-                    grad_pairs<T, S>(s, m, ne, rc, inv_rc, rc2d, lane < n ? s.queue[lane] : 0u, n, lane);
+                for (int cb = 0; cb < pr.ncand || (fin && cb == 0); cb += 32) {
+                    int j, k;
+                    bool ok = pr.get(j, k);
+                    if (ok) {
+                        const V4<T> a = s.nb[j], bb = s.nb[k];
+                        const T ex = bb.x - a.x, ey = bb.y - a.y, ez = bb.z - a.z;
+                        ok = ex * ex + ey * ey + ez * ez < rc2;
+                    }
+                    pr.next();
+                    const unsigned bal = __ballot_sync(kFull, ok);
+                    if (ok)
+                        s.queue[(qh + qn + __popc(bal & lanemask_lt())) & 63] =
+                            (unsigned)j | ((unsigned)k << 10) | ((unsigned)t << 20);
+                    qn += __popc(bal);
                     __syncwarp();
-                    const int rem = qlen - n;
-                    unsigned v = 0;
-                    if (lane < rem) v = s.queue[n + lane];
-                    __syncwarp();
-                    if (lane < rem) s.queue[lane] = v;
-                    __syncwarp();
-                    qlen = rem;
+                    if (qn >= 32 || (fin && qn > 0)) {
+                        const int n = qn < 32 ? qn : 32;
+                        grad_pairs<T, S, kB>(s, m, ne, rc, inv_rc, rc2d, lane < n ? s.queue[(qh + lane) & 63] : 0u, n, lane);
+                        __syncwarp();
+                        qh += n;
+                        qn -= n;
+                    }
                 }
             }
-        }
         }
         __syncwarp();
         T* gent = Buf<T>::gent(b);
         T sx = 0, sy = 0, sz = 0;
         T v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         for (int t = lane; t < Ms; t += 32) {
-            const V4<T> g{s.gx[t], s.gy[t], s.gz[t], (T)0};
+            V4<T> g{s.gx[t], s.gx[s.gst + t], s.gx[2 * s.gst + t], (T)0};
+#pragma unroll
+            for (int q = 1; q < kCopies; ++q) {
+                g.x += s.gx[3 * q * s.gst + t];
+                g.y += s.gx[(3 * q + 1) * s.gst + t];
+                g.z += s.gx[(3 * q + 2) * s.gst + t];
+            }
             const V4<T> d = s.nb[t];
             const size_t e = (size_t)s.ent[t];
             gent[3 * e] = g.x;
@@ -1203,56 +1363,77 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(T) == 4 ? 8 : 5) k_sfg_fas
 
 int nsm() { return device_sm_count(); }
 
+constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory of a block
+
 template <typename K>
 void set_smem(K kernel, size_t smem) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // always the same value: contexts on other threads launch the same kernel
+    // with other sizes, and one's smaller limit must not meet another's launch
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
 }
 
 // Shared memory per warp grows with the largest neighbour count of the
 // batch, and it sets how many warps an SM holds.  Atoms with at most `split`
-// neighbours (64 by default: about 98 % in the dense workloads) run in a
-// launch sized for that count; the rest follow in a second launch sized for
-// the batch maximum.  Each atom is evaluated once, by the same code.  The
-// split and the persistent grid (blocks per SM) are the knobs of the plans'
-// autotuner (Batch::sf_split, Batch::sf_blocks_per_sm).
-constexpr int kSplitCount = 64;
+// neighbours run in a launch sized for that count, which lists the others;
+// those follow in a second launch sized for the batch maximum.  Each atom is
+// evaluated once, by the same code.  (A second launch that searched all atoms
+// for its own took 0.3 ms of a 1024-structure step, nearly all of it latency.)
+// The split and the persistent grid (blocks per SM) are the knobs of the
+// plans' autotuner (Batch::sf_split, Batch::sf_blocks_per_sm).
 constexpr int kBlocksPerSm = 32;
 
-template <typename T, class S>
-int run_spec(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
+template <typename T, class S, bool kB>
+int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
     const int mfull = b.mmax > 0 ? ((b.mmax + 31) / 32) * 32 : 32;
-    int split = b.sf_split > 0 ? b.sf_split : b.sf_split < 0 ? mfull : kSplitCount;
+    auto warp_bytes = [&](int mm) { return fast_warp_bytes<T, S>(mm, m.nel, m.g2max, m.nblk, grad); };
+    // default split: the largest count at which the blocks the registers
+    // allow still fit (1 KB of every block is the system's)
+    const int resident = grad ? kBlocksG<T> : kBlocksV<T>;
+    int fitting = 32;
+    while (fitting + 4 <= 1024 && (warp_bytes(fitting + 4) * kWarps + 1024) * resident <= 228 * 1024) fitting += 4;
+    int split = b.sf_split > 0 ? (b.sf_split + 3) / 4 * 4 : b.sf_split < 0 ? mfull : fitting;
     const int per_sm = b.sf_blocks_per_sm > 0 ? b.sf_blocks_per_sm : kBlocksPerSm;
     if (b.sf_split == 0 && mfull > split) {
         // a batch whose warps all fit on the GPU at the full size needs no
         // second launch (same code per atom: same results)
-        const size_t blk = fast_warp_bytes<T>(mfull, m.g2max, m.nblk, S::P, grad) * kWarps;
-        const int fit = std::min<int>(sizeof(T) == 4 ? (grad ? 8 : 7) : 4, (int)((227u * 1024u) / blk));
+        const int fit = std::min<int>(resident, (int)(kSmemMax / (warp_bytes(mfull) * kWarps)));
         if ((long long)b.natoms <= (long long)nsm() * fit * kWarps) split = mfull;
     }
     int L = 0;
-    auto go = [&](int mm, int mlo, int last) {
-        const size_t smem = fast_warp_bytes<T>(mm, m.g2max, m.nblk, S::P, grad) * kWarps;
-        int blocks = (b.natoms + kWarps - 1) / kWarps;
+    auto go = [&](int mm, int part) {
+        // four warps a block, fewer where so many neighbours do not fit
+        int nw = kWarps;
+        while (nw > 1 && warp_bytes(mm) * nw > kSmemMax) nw >>= 1;
+        const size_t smem = warp_bytes(mm) * nw;
+        int blocks = (b.natoms + nw - 1) / nw;
         const int cap = nsm() * per_sm;
         if (blocks > cap) blocks = cap;
         if (blocks < 1) blocks = 1;
         if (grad) {
-            set_smem(k_sfg_fast<T, S>, smem);
-            k_sfg_fast<T, S><<<blocks, 32 * kWarps, smem, st>>>(b, m, mm, mlo, last);
+            set_smem(k_sfg_fast<T, S, kB>, smem);
+            k_sfg_fast<T, S, kB><<<blocks, 32 * nw, smem, st>>>(b, m, mm, part);
         } else {
-            set_smem(k_sfv_fast<T, S>, smem);
-            k_sfv_fast<T, S><<<blocks, 32 * kWarps, smem, st>>>(b, m, mm, mlo, last);
+            set_smem(k_sfv_fast<T, S, kB>, smem);
+            k_sfv_fast<T, S, kB><<<blocks, 32 * nw, smem, st>>>(b, m, mm, part);
         }
         ++L;
     };
     if (mfull > split) {
-        go(split, -1, 0);
-        go(mfull, split, 1);
+        cudaMemsetAsync(b.wide + (grad ? 1 : 0), 0, sizeof(int), st);
+        go(split, kPartFirst);
+        go(mfull, kPartWide);
     } else {
-        go(mfull, -1, 1);
+        go(mfull, kPartAll);
     }
     return L;
+}
+
+// FP64: the form without exponential range tests where the potential allows it
+template <typename T, class S>
+int run_spec(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
+    if constexpr (sizeof(T) == 8)
+        if (m.exp_bounded) return run_form<T, S, true>(b, m, grad, st);
+    return run_form<T, S, false>(b, m, grad, st);
 }
 
 template <typename T>
@@ -1270,9 +1451,15 @@ int run_any(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
 
 }  // namespace
 
+// The bytes per warp by which the pipeline limits the neighbour count (times
+// 4 against 220 KB): vectors and factors of 4 values, three accumulators, the
+// entry and the element of each neighbour, and the weight tensors.
 size_t sf_fast_smem_per_warp(int mmax, int g2max, int nblk, int P, bool grad, bool fp32) {
-    const int mm = mmax > 0 ? ((mmax + 31) / 32) * 32 : 32;
-    return fp32 ? fast_warp_bytes<float>(mm, g2max, nblk, P, grad) : fast_warp_bytes<double>(mm, g2max, nblk, P, grad);
+    const size_t mm = mmax > 0 ? ((mmax + 31) / 32) * 32 : 32, w = fp32 ? 4 : 8;
+    size_t n = 2 * a16(4 * w * mm) + a16(mm) + 64 * sizeof(unsigned) + a16(sizeof(int) * (kMaxEl + 1)) + a16(sizeof(int) * kMaxEl);
+    if (grad) n += 3 * a16(w * mm) + a16(sizeof(int) * mm) + a16(w * g2max) + 2 * a16(w * nblk * P);
+    else n += a16(w * 32 * (P + 1)) + (fp32 ? a16(sizeof(double4) * mm) : 0);
+    return n;
 }
 
 int launch_sf_values_fast(const Batch& b, const DevModel& m, bool fp32, cudaStream_t st) {

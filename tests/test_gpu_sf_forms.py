@@ -1,0 +1,123 @@
+"""The product-space symmetry-function kernels over the forms their launch
+accepts, against the FP64 oracle: grids of one, two and four etas and up to
+eight zetas (accumulator tiles, several passes over the partner elements),
+exponents inside and beyond the range of the form without range tests, centre
+elements without functions for some element pairs; centres without pairs,
+with more neighbours than the first launch takes and with more pairs than the
+pair list holds.
+
+FP64: |dE| <= 1e-10 |E|, max |dF|, |d dE/dh| <= 1e-9 times the largest force
+(at least 1).  Mixed precision: 1e-4 of the largest force, the FP32 rounding
+(6e-8) of some 500 pairs' terms through networks with summed weights of ~10."""
+import itertools
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SYM = {1: "H", 6: "C", 7: "N", 53: "I", 82: "Pb"}
+
+
+def write_potential(d, etas, zetas, missing=False, radial=(0.002, 0.05, 0.4), rs=(0.0, 1.5, 4.0), seed=5):
+    """5 elements, G2 for every neighbour element and G4 on the grid; with
+    `missing`, N centres have no functions for pairs with I and Pb centres no
+    radial functions for C."""
+    rows, n = [], {}
+    for c in SYM:
+        k = 0
+        for e in SYM:
+            for eta, r in zip(radial, rs):
+                if not (missing and c == 82 and e == 6):
+                    rows.append(f"symfunction_short {SYM[c]} 2 {SYM[e]} {eta:.6f} {r:.4f} 12.0000")
+                    k += 1
+        for a, b in itertools.combinations_with_replacement(SYM, 2):
+            if missing and c == 7 and 53 in (a, b):
+                continue
+            for eta in etas:
+                for lam in (-1.0, 1.0):
+                    for z in zetas:
+                        rows.append(f"symfunction_short {SYM[c]} 3 {SYM[a]} {SYM[b]} {eta:.6f} {lam:.1f} {z:.1f} 12.0000")
+                        k += 1
+        n[c] = k
+    (d / "input.nn").write_text("\n".join([
+        "number_of_elements 5", "elements " + " ".join(SYM.values()), "global_hidden_layers_short 2",
+        "global_nodes_short 9 7", "global_activation_short t t l", "cutoff_type 2", "scale_symmetry_functions",
+        "center_symmetry_functions"] + rows) + "\n")
+    rng = np.random.default_rng(seed)
+    sc = [f"{ie + 1} {k + 1} 0.0 {rng.uniform(3, 9):.6f} {rng.uniform(0, 1):.6f}" for ie, z in enumerate(SYM)
+          for k in range(n[z])]
+    (d / "scaling.data").write_text("\n".join(sc) + "\n-1.0 1.0\n")
+    for z in SYM:
+        v = []
+        for i, o in ((n[z], 9), (9, 7), (7, 1)):
+            v += list(rng.normal(0, 1 / np.sqrt(i), i * o + o))
+        (d / f"weights.{z:03d}.data").write_text("\n".join(f"{x:.12e}" for x in v) + "\n")
+
+
+def structures(W):
+    rng = np.random.default_rng(3)
+    dense = W.strain(W.supercell(W.abx3_cell(), (2, 2, 2)), -0.2 * np.eye(3))  # ~100 neighbours, ~2,000 pairs
+    out = [W.strain(W.supercell(W.abx3_cell(), (2, 1, 1)), rng.uniform(-0.05, 0.05, (3, 3))), dense]
+    for s in out:
+        s["pos"] = s["pos"] + rng.normal(0, 0.1, s["pos"].shape)
+    # centres with no pair, one neighbour, three neighbours
+    out.append({"Z": np.array([7, 53, 6, 1], np.int32), "lat": None,
+                "pos": np.array([[0.0, 0, 0], [4, 1, 0.5], [1, 11.2, 2], [7, 3, 13.5]])})
+    out.append({"Z": np.array([82, 1, 53, 1, 7], np.int32), "lat": None,
+                "pos": np.array([[0.0, 0, 0], [3, 1, 0.2], [1, 3, 2.5], [-2, 2, 4], [2.5, -2, -3]])})
+    return out
+
+
+@pytest.mark.parametrize("etas, zetas, missing", [
+    ((0.001, 0.01), (1, 2, 4, 16), False),
+    ((0.001, 0.01), (1, 2, 4, 16), True),
+    ((0.004,), (1, 4), True),
+    ((0.003, 0.3), (1, 3, 5, 6), False),
+    ((0.001, 0.004, 0.02, 0.2), (1, 2, 6, 9), True),
+    ((0.002, 0.009), (1, 2, 3, 4, 5, 8, 12, 16), True),
+])
+def test_forms_against_oracle(pkg, orc, W, tmp_path, etas, zetas, missing):
+    from hdnnp_b200 import engine
+
+    write_potential(tmp_path, etas, zetas, missing)
+    model = orc.Model(str(tmp_path))
+    pot = engine.Hdnnp.from_runner(str(tmp_path))
+    try:
+        pot.set_option("small_eval", 0)
+        structs = structures(W)
+        for prec, lim in ((engine.HDNNP_PREC_FP64, 1e-9), (engine.HDNNP_PREC_MIXED, 1e-4)):
+            pot.set_precision(prec)
+            out = pot.eval_batch(structs)
+            at = 0
+            for k, s in enumerate(structs):
+                ref = model.eval(s["Z"], s["pos"], s["lat"])
+                n = len(s["Z"])
+                top = max(1.0, np.abs(ref["forces"]).max())
+                assert abs(out["energy"][k] - ref["energy"]) <= (1e-10 if lim == 1e-9 else 1e-5) * max(1.0, abs(ref["energy"]))
+                assert np.abs(out["forces"][at:at + n] - ref["forces"]).max() <= lim * top
+                if s["lat"] is not None:
+                    d = out["dEdLat"][9 * k:9 * k + 9].reshape(3, 3, order="F") - ref["dEdLat"]
+                    assert np.abs(d).max() <= lim * max(1.0, np.abs(ref["dEdLat"]).max())
+                at += n
+    finally:
+        pot.close()
+
+
+def test_forms_need_no_list(pkg, W, tmp_path):
+    """A structure evaluated in one launch, and split into launches by
+    neighbour count, bit for bit."""
+    from hdnnp_b200 import engine
+
+    write_potential(tmp_path, (0.001, 0.01), (1, 2, 4, 16))
+    pot = engine.Hdnnp.from_runner(str(tmp_path))
+    try:
+        s = structures(W)[1]
+        res = []
+        for split in (-1, 32, 64, 97):
+            pot.set_option("sf_split", split)
+            res.append(pot.energy_and_forces(engine.AtStruct(s["Z"], s["pos"], s["lat"]), dEdLat=True))
+        for r in res[1:]:
+            assert r[0] == res[0][0] and np.array_equal(r[1], res[0][1]) and np.array_equal(r[2], res[0][2])
+    finally:
+        pot.close()
