@@ -110,25 +110,71 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// shared memory of k_mlp_split in doubles: hidden weights with odd row
-// strides, activations/deltas [2][8][kDS], act'(c_l) [L][8][kDS], layer-1
-// partial sums [8 warps][8][kDS]
-__host__ __device__ inline int split_hidden_doubles(const DevModel& m) {
-    int n = 0;
-    for (int l = 1; l < m.nlayers; ++l) n += m.width[l] * (m.width[l + 1] | 1);
-    return (n + 1) & ~1;  // what follows starts on a 16-byte boundary
+// The later layers' weights in shared memory, layer by layer the fragments of
+// the forward product ([ks][nt][32], B[k][n] = W[n][k]) and of the backward
+// product (B[k][n] = W[k][n]), zero-padded; doubles they take.
+__host__ __device__ inline int hidden_doubles(const DevModel& m) {
+    int h = 0;
+    for (int l = 1; l < m.nlayers; ++l) {
+        const int wi = m.width[l], wo = m.width[l + 1];
+        h += (((wi + 3) >> 2) * ((wo + 7) >> 3) + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
+    }
+    return h;
 }
+__device__ __forceinline__ void stage_hidden(const DevModel& m, int e, double* h, int tid, int nthreads) {
+    const int L = m.nlayers;
+    for (int l = 1; l < L; ++l) {
+        const int wi = m.width[l], wo = m.width[l + 1];
+        const double* W = m.w + m.w_off[e * L + l];  // [wo][wi]
+        for (int dir = 0; dir < 2; ++dir) {
+            const int kk = dir ? wo : wi, nn = dir ? wi : wo;
+            const int NT = (nn + 7) >> 3, nf = ((kk + 3) >> 2) * NT * 32;
+            for (int idx = tid; idx < nf; idx += nthreads) {
+                const int t = idx & 31, f = idx >> 5, n = (f % NT) * 8 + (t >> 2), k = 4 * (f / NT) + (t & 3);
+                if (n < nn && k < kk) cp_async8(h + idx, W + (dir ? (size_t)k * wi + n : (size_t)n * wi + k));
+                else h[idx] = 0.0;
+            }
+            h += nf;
+        }
+    }
+}
+
+// C[8 x 8 NT] = A[8 x k] B: NC n-tiles from n0 on, the A fragments read from
+// the rows at `rows` (columns beyond k as zero), the B fragments [ks][nt][32]
+// at `B`, both in shared memory.
+template <int NC>
+__device__ __forceinline__ void rows_gemm(double (&acc)[NC][2], const double* rows, int k, const double* B, int NT, int n0,
+                                          int r, int q, int lane) {
+#pragma unroll
+    for (int nt = 0; nt < NC; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+    const int KS = (k + 3) >> 2;
+#pragma unroll 2
+    for (int ks = 0; ks < KS; ++ks) {
+        const double a = 4 * ks + q < k ? rows[r * kDS + 4 * ks + q] : 0.0;
+#pragma unroll
+        for (int nt = 0; nt < NC; ++nt)
+            if (n0 + nt < NT) dmma(acc[nt], a, B[(ks * NT + n0 + nt) * 32 + lane]);
+    }
+}
+
+// Pairs of k-steps (8 consecutive inputs; step v of pair p takes 8 p + 2 q + v
+// in fragment column q) whose products are summed on their own: both kernels
+// add layer 1 in kDW such segments, in order, so that an atom's result does
+// not depend on which of them evaluates its batch.
+__device__ __forceinline__ int segment_pairs(int nin) { return (((nin + 7) >> 3) + kDW - 1) / kDW; }
+
+// shared memory of k_mlp_split in doubles: later layers, activations or
+// deltas [8][kDS], act'(c_l) [L][8][kDS], layer-1 segments [8][8][kDS]
 __host__ __device__ inline int split_doubles(const DevModel& m) {
-    return split_hidden_doubles(m) + (2 + m.nlayers + kDW) * kDR * kDS;
+    return hidden_doubles(m) + (1 + m.nlayers + kDW) * kDR * kDS;
 }
 
 // Bound by the latency of one tile's chain: element and atom lookup, G and
-// W1 loads, the layers, dE/dG.  The 8 warps take 1/8 of layer 1's k-steps
-// each (partial sums added in warp order) and every 8th pair of dE/dG
-// columns; a thread owns one (atom, neuron) of the hidden layers, whose
-// weights arrive in shared memory while layer 1 multiplies.  Cold, a warp
-// per tile with all of it in one chain took 113 us for the 768-atom cell
-// (96 tiles).
+// W1 loads, the layers, dE/dG.  Each of the 8 warps takes a segment of layer
+// 1, an n-tile of the later layers (four warps; their weights arrive in shared
+// memory while layer 1 multiplies) and every 8th pair of dE/dG columns.  Cold,
+// a warp per tile with all of it in one chain took 113 us for the 768-atom
+// cell (96 tiles).
 __global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
     extern __shared__ __align__(16) double dsm[];
     const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
@@ -145,19 +191,11 @@ __global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
         tile -= nt;
     }
     if (e < 0) return;  // uniform per block
-    double* hw = dsm;
-    double* yb = hw + split_hidden_doubles(m);  // two rotating row sets
-    double* da = yb + 2 * kDR * kDS;
+    double* h = dsm;
+    double* yrow = h + hidden_doubles(m);
+    double* da = yrow + kDR * kDS;
     double* part = da + L * kDR * kDS;
-    {
-        double* dst = hw;
-        for (int l = 1; l < L; ++l) {
-            const int win = m.width[l], wout = m.width[l + 1], st = wout | 1;
-            const double* WT = m.wt + m.w_off[e * L + l];  // [win][wout]
-            for (int idx = tid; idx < win * wout; idx += 32 * kDW) cp_async8(dst + (idx / wout) * st + idx % wout, WT + idx);
-            dst += win * st;
-        }
-    }
+    stage_hidden(m, e, h, tid, 32 * kDW);
     const int r = lane >> 2, q = lane & 3;
     const int atom = r < cnt ? b.el_atoms[t0 + r] : -1;
     const int nin = m.nin_el[e], nsf = m.nsf_max, H1 = m.width[1];
@@ -166,16 +204,26 @@ __global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
         const double* grow = atom >= 0 ? b.G + (size_t)atom * nsf : nullptr;
-        const double* F = m.dm_fwd + m.dm_off_f[e] + lane;  // [ks][nt][32]
-        const int KS = (nin + 3) >> 2, per = (KS + kDW - 1) / kDW;
-        const int k0 = wib * per, k1 = min(KS, k0 + per);
+        const int KS = (nin + 3) >> 2, KP = (nin + 7) >> 3, per = segment_pairs(nin);
+        // [ks][nt][32]: this lane's inputs 2 q, 2 q + 1 of a pair lie in k-step
+        // 2 p + q/2
+        const double* F = m.dm_fwd + m.dm_off_f[e] + (lane & ~3) + ((2 * q) & 3);
+        const int p0 = wib * per, p1 = min(KP, p0 + per);
 #pragma unroll 5
-        for (int ks = k0; ks < k1; ++ks) {
-            const int k = 4 * ks + q;
-            const double a = (grow && k < nin) ? __ldg(grow + k) : 0.0;
+        for (int p = p0; p < p1; ++p) {
+            const int k = 8 * p + 2 * q, ks = 2 * p + (q >> 1);
+            double a[2], bf[4][2];
+#pragma unroll
+            for (int v = 0; v < 2; ++v) a[v] = (grow && k + v < nin) ? __ldg(grow + k + v) : 0.0;
             const double* f = F + (size_t)ks * 128;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], a, __ldg(f + nt * 32));
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) bf[nt][v] = ks < KS ? __ldg(f + nt * 32 + v) : 0.0;
+#pragma unroll
+            for (int v = 0; v < 2; ++v)
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], a[v], bf[nt][v]);
         }
         double* pw = part + wib * kDR * kDS + r * kDS + 2 * q;
 #pragma unroll
@@ -183,62 +231,63 @@ __global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
     }
     cp_async_wait();
     __syncthreads();
-    // thread = (atom wib, neuron lane) from here to the deltas
-    const int row = wib * kDS + lane;
-    if (lane < H1) {
-        double c = part[row];
+    {
+        const int row = wib * kDS + lane;  // (atom, neuron)
+        if (lane < H1) {
+            double c = part[row];
 #pragma unroll
-        for (int w = 1; w < kDW; ++w) c += part[w * kDR * kDS + row];
-        c += m.b[m.b_off[e * L] + lane];
-        const double y = act_f(m.act[0], c);
-        yb[row] = y;
-        da[row] = act_d(m.act[0], c, y);
-    }
-    __syncwarp();
-    const double* W = hw;
-    for (int l = 1; l < L; ++l) {
-        const int win = m.width[l], wout = m.width[l + 1], st = wout | 1;
-        const double* yin = yb + ((l - 1) & 1) * kDR * kDS + wib * kDS;
-        if (lane < wout) {
-            double c = 0.0;
-#pragma unroll 5
-            for (int i = 0; i < win; ++i) c += W[i * st + lane] * yin[i];
-            c += m.b[m.b_off[e * L + l] + lane];
-            const double y = act_f(m.act[l], c);
-            yb[(l & 1) * kDR * kDS + row] = y;
-            da[l * kDR * kDS + row] = act_d(m.act[l], c, y);
+            for (int w = 1; w < kDW; ++w) c += part[w * kDR * kDS + row];
+            c += m.b[m.b_off[e * L] + lane];
+            const double y = act_f(m.act[0], c);
+            const double d = act_d(m.act[0], c, y);
+            yrow[row] = L > 1 ? y : d;
+            da[row] = d;
+            if (L == 1 && lane == 0 && wib < cnt) b.atE[b.el_atoms[t0 + wib]] = y + m.atom_energy[e];
         }
-        W += win * st;
-        __syncwarp();
-    }
-    if (lane == 0 && wib < cnt)
-        b.atE[b.el_atoms[t0 + wib]] = yb[((L - 1) & 1) * kDR * kDS + row] + m.atom_energy[e];
-    __syncwarp();
-    // deltas in the rotating rows (gradOut = 1)
-    double* dcur = yb;
-    double* dnext = yb + kDR * kDS;
-    const double* dl = da + (L - 1) * kDR * kDS + row;  // act'(c_l) of this thread's neuron
-    if (lane < m.width[L]) dcur[row] = *dl;
-    __syncwarp();
-    for (int l = L - 1; l >= 1; --l) {
-        const int win = m.width[l], wout = m.width[l + 1], st = wout | 1;
-        W -= win * st;
-        dl -= kDR * kDS;
-        if (lane < win) {
-            double s = 0.0;
-#pragma unroll 5
-            for (int o = 0; o < wout; ++o) s += dcur[wib * kDS + o] * W[lane * st + o];
-            dnext[row] = s * *dl;
-        }
-        __syncwarp();
-        double* t = dcur;
-        dcur = dnext;
-        dnext = t;
     }
     __syncthreads();
+    // later layers and the deltas back to layer 1: a warp per n-tile
+    for (int l = 1; l < L; ++l) {
+        const int wi = m.width[l], wo = m.width[l + 1], NT = (wo + 7) >> 3;
+        double acc[1][2];
+        if (wib < NT) rows_gemm(acc, yrow, wi, h, NT, wib, r, q, lane);
+        h += (((wi + 3) >> 2) * NT + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
+        __syncthreads();
+        if (wib < NT)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int col = wib * 8 + 2 * q + v;
+                if (col < wo) {
+                    const double c = acc[0][v] + m.b[m.b_off[e * L + l] + col];
+                    const double y = act_f(m.act[l], c);
+                    const double d = act_d(m.act[l], c, y);
+                    yrow[r * kDS + col] = l + 1 < L ? y : d;  // gradOut = 1
+                    da[(l * kDR + r) * kDS + col] = d;
+                    if (l + 1 == L && atom >= 0 && col == 0) b.atE[atom] = y + m.atom_energy[e];
+                }
+            }
+        __syncthreads();
+    }
+    const double* dl = da + (L - 1) * kDR * kDS;
+    for (int l = L - 1; l >= 1; --l) {
+        const int wi = m.width[l], wo = m.width[l + 1], NT = (wi + 7) >> 3;
+        const int nb = ((wo + 3) >> 2) * NT * 32;
+        dl -= kDR * kDS;
+        double acc[1][2];
+        if (wib < NT) rows_gemm(acc, yrow, wo, h - nb, NT, wib, r, q, lane);
+        h -= nb + ((wi + 3) >> 2) * ((wo + 7) >> 3) * 32;
+        __syncthreads();
+        if (wib < NT)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int col = wib * 8 + 2 * q + v;
+                if (col < wi) yrow[r * kDS + col] = acc[0][v] * dl[r * kDS + col];
+            }
+        __syncthreads();
+    }
     double afr[kDH / 4];
 #pragma unroll
-    for (int ks = 0; ks < kDH / 4; ++ks) afr[ks] = (4 * ks + q < H1) ? dcur[r * kDS + 4 * ks + q] : 0.0;
+    for (int ks = 0; ks < kDH / 4; ++ks) afr[ks] = (4 * ks + q < H1) ? yrow[r * kDS + 4 * ks + q] : 0.0;
     const double* Bw = m.dm_bwd + m.dm_off_b[e] + lane;  // [nb][ks][32]
     const int KB = (H1 + 3) >> 2, NB = (nin + 7) >> 3;
     for (int nb = 2 * wib; nb < NB; nb += 2 * kDW) {
@@ -278,32 +327,10 @@ __host__ __device__ inline DmmaLayout dmma_layout(const DevModel& m, int nin) {
     o.f1 = 0;
     o.b1 = o.f1 + ((nin + 7) >> 3) * 8 * 32;
     o.hid = o.b1 + ((nin + 7) >> 3) * ((H1 + 3) >> 2) * 32;
-    int h = 0;
-    for (int l = 1; l < L; ++l) {
-        const int wi = m.width[l], wo = m.width[l + 1];
-        h += (((wi + 3) >> 2) * ((wo + 7) >> 3) + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
-    }
-    o.bias = o.hid + h;
+    o.bias = o.hid + hidden_doubles(m);
     o.warps = o.bias + L * kDH;
     o.total = o.warps + kRW * L * kDR * kDS;
     return o;
-}
-
-// C[8 x 8 NT] += A[8 x 4 KS] B with the A fragments read from the rows at
-// `rows` and the B fragments [ks][nt][32] at `B`, both in shared memory;
-// columns of A beyond `k` read as zero.
-__device__ __forceinline__ void rows_gemm(double (&acc)[4][2], const double* rows, int k, const double* B, int NT, int r,
-                                          int q, int lane) {
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
-    const int KS = (k + 3) >> 2;
-#pragma unroll 2
-    for (int ks = 0; ks < KS; ++ks) {
-        const double a = 4 * ks + q < k ? rows[r * kDS + 4 * ks + q] : 0.0;
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-            if (nt < NT) dmma(acc[nt], a, B[(ks * NT + nt) * 32 + lane]);
-    }
 }
 
 // Bound by the FP64 tensor cores (about 590 m8n8k4 per tile of a
@@ -337,7 +364,7 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
         const int s0 = max(first, base) - base, s1 = min(end, base + nte) - base;
         base += nte;
         if (s0 >= s1) continue;  // uniform per block
-        const int nin = m.nin_el[e], KP = (nin + 7) >> 3, NB = KP;
+        const int nin = m.nin_el[e], KP = (nin + 7) >> 3, NB = KP, per = segment_pairs(nin);
         __syncthreads();  // the previous element's weights are no longer read
         {
             // [2 p + v][nt][t] = W1[8 nt + t/4][8 p + 2 (t%4) + v], from the
@@ -354,23 +381,7 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
             }
             for (int idx = tid; idx < NB * KB * 32; idx += 32 * kRW)
                 cp_async8(dsm + lo.b1 + idx, m.dm_bwd + m.dm_off_b[e] + idx);
-            double* h = dsm + lo.hid;
-            for (int l = 1; l < L; ++l) {
-                const int wi = m.width[l], wo = m.width[l + 1];
-                const double* W = m.w + m.w_off[e * L + l];  // [wo][wi]
-                const int NT = (wo + 7) >> 3, nf = ((wi + 3) >> 2) * NT * 32;
-                for (int idx = tid; idx < nf; idx += 32 * kRW) {
-                    const int t = idx & 31, n = ((idx >> 5) % NT) * 8 + (t >> 2), k = 4 * ((idx >> 5) / NT) + (t & 3);
-                    h[idx] = (n < wo && k < wi) ? W[(size_t)n * wi + k] : 0.0;
-                }
-                h += nf;
-                const int NT2 = (wi + 7) >> 3, nb = ((wo + 3) >> 2) * NT2 * 32;
-                for (int idx = tid; idx < nb; idx += 32 * kRW) {
-                    const int t = idx & 31, n = ((idx >> 5) % NT2) * 8 + (t >> 2), k = 4 * ((idx >> 5) / NT2) + (t & 3);
-                    h[idx] = (k < wo && n < wi) ? W[(size_t)k * wi + n] : 0.0;
-                }
-                h += nb;
-            }
+            stage_hidden(m, e, dsm + lo.hid, tid, 32 * kRW);
             for (int idx = tid; idx < L * kDH; idx += 32 * kRW) {
                 const int l = idx / kDH, n = idx % kDH;
                 dsm[lo.bias + idx] = n < m.width[l + 1] ? m.b[m.b_off[e * L + l] + n] : 0.0;
@@ -409,9 +420,10 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
         for (int tile = s0 + wib; tile < s1; tile += kRW) {
             const int atom = atom_n;
             atom_n = atom_of(tile + kRW);
-            double acc[4][2];
+            double acc[4][2], sum[4][2];  // a segment's products, the segments before it
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+            for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = sum[nt][0] = sum[nt][1] = 0.0;
+            int left = per;
             for (int p0 = 0; p0 < KP; p0 += kCh) {
                 const bool more = p0 + kCh < KP;
                 const int an_atom = more ? atom : atom_n, an_p = more ? p0 + kCh : 0;
@@ -423,16 +435,30 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
                         for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], an[i].x, f[nt * 32]);
 #pragma unroll
                         for (int nt = 0; nt < 4; ++nt) dmma(acc[nt], an[i].y, f[128 + nt * 32]);
+                        if (--left == 0) {
+                            left = per;
+#pragma unroll
+                            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                                for (int v = 0; v < 2; ++v) {
+                                    sum[nt][v] += acc[nt][v];
+                                    acc[nt][v] = 0.0;
+                                }
+                        }
                     }
                     load(an_atom, an_p + i, an[i]);
                 }
             }
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) acc[nt][v] = sum[nt][v] + acc[nt][v];
             const double* h = dsm + lo.hid;
             for (int l = 0; l < L; ++l) {
                 const int wo = m.width[l + 1], NT = (wo + 7) >> 3;
                 if (l > 0) {
                     const int wi = m.width[l];
-                    rows_gemm(acc, yrow, wi, h, NT, r, q, lane);
+                    rows_gemm(acc, yrow, wi, h, NT, 0, r, q, lane);
                     h += (((wi + 3) >> 2) * NT + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
                     __syncwarp();
                 }
@@ -460,7 +486,7 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
             for (int l = L - 1; l >= 1; --l) {
                 const int wi = m.width[l], wo = m.width[l + 1], NT = (wi + 7) >> 3;
                 const int nb = ((wo + 3) >> 2) * NT * 32;
-                rows_gemm(acc, yrow, wo, h - nb, NT, r, q, lane);
+                rows_gemm(acc, yrow, wo, h - nb, NT, 0, r, q, lane);
                 h -= nb + ((wi + 3) >> 2) * ((wo + 7) >> 3) * 32;
                 __syncwarp();
 #pragma unroll
@@ -542,11 +568,13 @@ void run_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
 // with one output and at most 8 layers (dm_ok, set with the fragments at
 // model upload).  The resident form needs an element's weights to fit in
 // shared memory and enough tiles to keep its warps busy: its time for one
-// tile is long (53 us from 4,500 atoms down, against 19-34 us of the split
-// form).  Measured for 280-25-25-1 networks, split / resident: 83 / 86 us at
-// 18,000 atoms, 137 / 141 at 36,000, 250 / 228 at 71,000; the line lies
-// between the last two.
-constexpr int kResidentTilesPerSm = 36;
+// tile is long (53 us from 4,500 atoms down, against 18-35 us of the split
+// form).  Measured for 280-25-25-1 networks, split / resident: 93 / 88 us at
+// 18,000 atoms, 156 / 145 at 36,000.  Both give an atom the same bits.
+constexpr int kResidentTilesPerSm = 16;
+// dynamic shared memory of a block; always set as the kernels' limit (contexts
+// on other threads may launch them with other sizes)
+constexpr int kSmemLimit = 227 * 1024;
 
 int launch_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     if (!m.dm_ok) {
@@ -557,14 +585,14 @@ int launch_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     for (int e = 0; e < m.nel; ++e) nin = nin > m.nin_el[e] ? nin : m.nin_el[e];
     const size_t rsm = (size_t)dmma_layout(m, nin).total * sizeof(double);
     const int nsm = device_sm_count();
-    if (rsm <= 227 * 1024 && b.natoms >= nsm * kResidentTilesPerSm * kDR) {
+    if (rsm <= (size_t)kSmemLimit && b.natoms >= nsm * kResidentTilesPerSm * kDR) {
         auto k = (m.nsf_max & 1) ? k_mlp_resident<false> : k_mlp_resident<true>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
         k<<<nsm, 32 * kRW, rsm, s>>>(b, m, nin);
         return 1;
     }
     const size_t smem = (size_t)split_doubles(m) * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_mlp_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k_mlp_split, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     k_mlp_split<<<b.natoms / kDR + m.nel + 1, 32 * kDW, smem, s>>>(b, m);
     return 1;
 }

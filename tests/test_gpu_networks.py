@@ -38,8 +38,8 @@ def layers(net, x):
 
 
 @pytest.mark.parametrize("pot_dir, natoms", [(EXAMPLE_DIR, 8), (EXAMPLE_DIR, 1), (ABX3_DIR, 7), (ABX3_DIR, 9),
-                                             (ABX3_DIR, 97), (PRZ_DIR, 65), (ABX3_DIR, 42611), (ABX3_DIR, 42630),
-                                             (PRZ_DIR, 42631)])
+                                             (ABX3_DIR, 97), (PRZ_DIR, 65), (ABX3_DIR, 18936), (ABX3_DIR, 18945),
+                                             (PRZ_DIR, 18951)])
 def test_networks(pkg, W, pot_dir, natoms):
     from hdnnp_b200 import engine
 
@@ -50,7 +50,7 @@ def test_networks(pkg, W, pot_dir, natoms):
         if pot_dir == EXAMPLE_DIR:
             s = W.read_xyz(EXAMPLE_DIR + "/input.xyz")
         else:
-            s = W.supercell(W.abx3_cell(), (17, 15, 14) if natoms > 1000 else (3, 3, 1))
+            s = W.supercell(W.abx3_cell(), (12, 12, 11) if natoms > 1000 else (3, 3, 1))
             s["pos"] = s["pos"] + rng.normal(0, 0.1, s["pos"].shape)
         Z, pos = s["Z"][:natoms], s["pos"][:natoms]
         pot.energy_and_forces(engine.AtStruct(Z, pos, s["lat"]))
@@ -65,5 +65,27 @@ def test_networks(pkg, W, pot_dir, natoms):
             e = e + e0[int(z) - 1]
             assert np.abs(E[m] - e).max() <= te + 4 * EPS * np.abs(e).max()
             assert np.abs(D[m][:, :n] - g).max() <= tg
+    finally:
+        pot.close()
+
+
+@pytest.mark.parametrize("pot_dir", [ABX3_DIR, PRZ_DIR])
+def test_alone_equals_in_the_large_batch(pkg, W, pot_dir):
+    """The per-tile and the weights-resident kernel give an atom the same bits."""
+    from hdnnp_b200 import engine
+
+    pot = engine.Hdnnp.from_runner(pot_dir)
+    try:
+        rng = np.random.default_rng(8)
+        small = W.strain(W.supercell(W.abx3_cell(), (2, 2, 1)), rng.uniform(-0.05, 0.05, (3, 3)))
+        small["pos"] = small["pos"] + rng.normal(0, 0.15, small["pos"].shape)
+        big = W.supercell(W.abx3_cell(), (12, 12, 11))
+        big["pos"] = big["pos"] + rng.normal(0, 0.1, big["pos"].shape)
+        alone = pot.eval_batch([small])
+        both = pot.eval_batch([big, small])
+        n = len(small["Z"])
+        assert both["energy"][1] == alone["energy"][0]
+        assert np.array_equal(both["forces"][-n:], alone["forces"])
+        assert np.array_equal(both["dEdLat"][9:], alone["dEdLat"])
     finally:
         pot.close()
