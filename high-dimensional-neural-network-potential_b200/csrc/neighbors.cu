@@ -43,9 +43,7 @@ __global__ void k_atom_struct(const StructInfo* info, int nstruct, int* sid) {
 }
 
 // K1: wrap into the cell, element index, cell id, per-cell counts.
-__global__ void k_wrap_bin(Batch b, DevModel m) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b.natoms) return;
+__device__ __forceinline__ void wrap_bin(const Batch& b, const DevModel& m, int i) {
     if (keep_list(b)) {
         // same translation as at the last build: distances to the listed images stay consistent
         for (int d = 0; d < 3; ++d) {
@@ -96,6 +94,11 @@ __global__ void k_wrap_bin(Batch b, DevModel m) {
     int cid = S.cell_off + (c0 * S.ngrid[1] + c1) * S.ngrid[2] + c2;
     b.cell_of[i] = cid;
     atomicAdd(&b.cell_cnt[cid], 1);
+}
+
+__global__ void k_wrap_bin(Batch b, DevModel m) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < b.natoms) wrap_bin(b, m, i);
 }
 
 __global__ void k_fill_cells(Batch b, int* cursor) {
@@ -378,6 +381,252 @@ __global__ void k_neighbours_warp(Batch b, DevModel m) {
     if (kMode != 1 && lane == 0) b.nei_cnt[i] = n;
 }
 
+// The padded-row pass with a warp per cell: the cell's atoms have the same
+// virtual cells, so their candidates (position with the image shift added,
+// index, shift and slab) are staged in shared memory once, in the reference's
+// order, and each atom of the cell is tested against 32 of them at a time; a
+// ballot gives the accepted ones their places in the row.  Same arithmetic
+// per candidate and same order as the other forms, so the rows and the slab
+// table are the same entry for entry.
+// Bound by instruction issue and L2 latency: a thread per atom walked ~330
+// candidates of cells of uneven occupancy with half its lanes idle (2.9 ms of
+// the 4096-structure step).
+constexpr int kCellWarps = 4;
+constexpr int kCellCap = 128;  // candidates staged at a time
+__global__ void __launch_bounds__(32 * kCellWarps) k_neighbours_cell(Batch b, DevModel m) {
+    __shared__ double4 cpos[kCellWarps][kCellCap];  // x, y, z; index | shift and slab << 32
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cell = blockIdx.x * kCellWarps + wib;
+    if (cell >= b.ncells || keep_list(b)) return;  // uniform per warp
+    const int a0 = b.cell_start[cell], na = b.cell_start[cell + 1] - a0;
+    if (na <= 0) return;
+    double4* cp = cpos[wib];
+    const StructInfo& S = b.info[b.sid[b.cell_atoms[a0]]];
+    const double rc = b.rc_list > 0.0 ? b.rc_list : m.max_rc, rc2 = rc * rc;
+    const int c = cell - S.cell_off;
+    const int ix = c / (S.ngrid[1] * S.ngrid[2]);
+    const int iy = (c / S.ngrid[2]) % S.ngrid[1];
+    const int iz = c % S.ngrid[2];
+    const double* h = S.h;
+    const int ny = 2 * S.nsearch[1] + 1, nz = 2 * S.nsearch[2] + 1;
+    const int nv = (2 * S.nsearch[0] + 1) * ny * nz, nslab = nv / nz;
+    const bool tabs = b.slab && nslab <= kMaxSlabs;
+    for (int g0 = 0; g0 < na; g0 += 32) {
+        // this lane's atom of the group and the entries found for it
+        const int ng = min(32, na - g0);
+        double xi = 0.0, yi = 0.0, zi = 0.0;
+        int i = -1, n = 0;
+        if (lane < ng) i = cand(b, a0 + g0 + lane, xi, yi, zi);
+        for (int v0 = 0; v0 < nv; v0 += 32) {
+            const int v = v0 + lane;
+            int p0 = 0, cnt = 0, dx = 0, dy = 0, dz = 0;
+            double lx = 0, ly = 0, lz = 0;
+            if (v < nv) {
+                int cx = ix + v / (ny * nz) - S.nsearch[0], cy = iy + (v / nz) % ny - S.nsearch[1],
+                    cz = iz + v % nz - S.nsearch[2];
+                bool inside = true;
+                if (cz < 0 || cz >= S.ngrid[2]) {
+                    inside = S.periodic;
+                    dz = wrap_cell(cz, S.ngrid[2]);
+                }
+                if (cy < 0 || cy >= S.ngrid[1]) {
+                    inside = inside && S.periodic;
+                    dy = wrap_cell(cy, S.ngrid[1]);
+                }
+                if (cx < 0 || cx >= S.ngrid[0]) {
+                    inside = inside && S.periodic;
+                    dx = wrap_cell(cx, S.ngrid[0]);
+                }
+                if (inside) {
+                    if (dz) { lx += h[6] * dz; ly += h[7] * dz; lz += h[8] * dz; }
+                    if (dy) { lx += h[3] * dy; ly += h[4] * dy; lz += h[5] * dy; }
+                    if (dx) { lx += h[0] * dx; ly += h[1] * dx; lz += h[2] * dx; }
+                    const int cc = S.cell_off + (cx * S.ngrid[1] + cy) * S.ngrid[2] + cz;
+                    p0 = b.cell_start[cc];
+                    cnt = b.cell_start[cc + 1] - p0;
+                }
+            }
+            int incl = cnt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += o;
+            }
+            const int off = incl - cnt, total = __shfl_sync(0xffffffffu, incl, 31);
+            const bool slab_start = tabs && v < nv && v % nz == 0;
+            const int sh = pack_shift(dx, dy, dz) | (tabs && v < nv ? (v / nz) << 24 : 0);
+            // candidates w0 .. w0 + T of these virtual cells at a time (once
+            // with T = 0 for the slab table)
+            for (int w0 = 0; w0 == 0 || w0 < total; w0 += kCellCap) {
+                const int T = min(kCellCap, total - w0);
+                __syncwarp();
+                for (int k = max(0, w0 - off); k < cnt && off + k < w0 + T; ++k) {
+                    double px, py, pz;
+                    const int j = cand(b, p0 + k, px, py, pz);
+                    cp[off + k - w0] = make_double4(px + lx, py + ly, pz + lz, __hiloint2double(sh, j));
+                }
+                __syncwarp();
+                // slabs that start in this window, or behind the last candidate
+                const bool mine = slab_start && off >= w0 && (off < w0 + kCellCap || w0 + kCellCap >= total);
+                for (int a = 0; a < ng; ++a) {
+                    const double x = __shfl_sync(0xffffffffu, xi, a), y = __shfl_sync(0xffffffffu, yi, a),
+                                 z = __shfl_sync(0xffffffffu, zi, a);
+                    const int ia = __shfl_sync(0xffffffffu, i, a);
+                    int na_ = __shfl_sync(0xffffffffu, n, a);
+                    int2* row = b.pad + (size_t)ia * b.pad_cap;
+                    int before = na_;  // entries before this lane's slab start
+                    for (int q0 = 0; q0 < T; q0 += 32) {
+                        const int q = q0 + lane;
+                        bool ok = false;
+                        int j = 0, sj = 0;
+                        if (q < T) {
+                            const double4 r = cp[q];
+                            j = __double2loint(r.w);
+                            sj = __double2hiint(r.w);
+                            const double ddx = x - r.x, ddy = y - r.y, ddz = z - r.z;
+                            ok = ddx * ddx + ddy * ddy + ddz * ddz < rc2 && !(j == ia && (sj & 0xffffff) == 0);
+                        }
+                        const unsigned bal = __ballot_sync(0xffffffffu, ok);
+                        const int at = na_ + __popc(bal & ((1u << lane) - 1u));
+                        if (ok && at < b.pad_cap) row[at] = make_int2(j, sj);
+                        if (mine) {
+                            const int upto = off - w0 - q0;  // candidates of this word before the slab
+                            before += upto >= 32 ? __popc(bal) : upto > 0 ? __popc(bal & ((1u << upto) - 1u)) : 0;
+                        }
+                        na_ += __popc(bal);
+                    }
+                    if (mine) b.slab[(size_t)ia * kSlabStride + v / nz] = (unsigned short)min(before, 0xffff);
+                    if (lane == a) n = na_;
+                }
+            }
+        }
+        if (lane < ng) {
+            b.nei_cnt[i] = n;
+            if (tabs) b.slab[(size_t)i * kSlabStride + nslab] = (unsigned short)min(n, 0xffff);
+        }
+    }
+}
+
+// ---------------------------------------------------------------- small batches
+// One block does what the chains of small kernels above do for a batch of at
+// most kSmallAtoms atoms, whose time is that of the launches: the cell stage
+// (clear, wrap and bin, scan, fill, sort, cell-ordered positions), the list
+// offsets (scan, largest count) with the capacity check, the element groups
+// (mlp.cu).
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallAtoms = 2048;
+constexpr int kSmallCells = 4096;
+
+// exclusive sum over the block's threads (1024) of v; *total: the sum of all
+__device__ __forceinline__ int block_exclusive(int v, int* wsum, int* total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        int t = wsum[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += y;
+        }
+        wsum[lane] = t;
+    }
+    __syncthreads();
+    *total = wsum[31];
+    return x - v + (w > 0 ? wsum[w - 1] : 0);
+}
+
+__global__ void __launch_bounds__(kSmallThreads) k_small_cells(Batch b, DevModel m) {
+    __shared__ int wsum[32];
+    __shared__ int start[kSmallCells + 1];
+    __shared__ int fill[kSmallCells];
+    __shared__ int atoms[kSmallAtoms];
+    const int tid = threadIdx.x;
+    if (keep_list(b)) {  // uniform
+        for (int i = tid; i < b.natoms; i += kSmallThreads) wrap_bin(b, m, i);
+        return;
+    }
+    for (int c = tid; c <= b.ncells; c += kSmallThreads) b.cell_cnt[c] = 0;
+    __syncthreads();
+    for (int i = tid; i < b.natoms; i += kSmallThreads) wrap_bin(b, m, i);
+    __syncthreads();
+    {
+        constexpr int kPer = kSmallCells / kSmallThreads;
+        int v[kPer], sum = 0, total;
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int c = tid * kPer + u;
+            v[u] = c < b.ncells ? atomicAdd(&b.cell_cnt[c], 0) : 0;
+            sum += v[u];
+        }
+        int at = block_exclusive(sum, wsum, &total);
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int c = tid * kPer + u;
+            if (c <= b.ncells && c < kSmallCells) {
+                start[c] = at;
+                b.cell_start[c] = at;
+                if (c < kSmallCells) fill[c] = 0;
+            }
+            at += v[u];
+        }
+        if (tid == 0) {
+            start[b.ncells] = total;
+            b.cell_start[b.ncells] = total;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < b.natoms; i += kSmallThreads) {
+        const int c = b.cell_of[i];
+        atoms[start[c] + atomicAdd(&fill[c], 1)] = i;
+    }
+    __syncthreads();
+    // deterministic order inside a cell: every atom to its rank
+    for (int p = tid; p < b.natoms; p += kSmallThreads) {
+        const int v = atoms[p], c = b.cell_of[v];
+        int r = start[c];
+        for (int q = start[c]; q < start[c + 1]; ++q) r += atoms[q] < v;
+        b.cell_atoms[r] = v;
+        if (b.posc)
+            b.posc[r] = make_double4(b.wpos[3 * v], b.wpos[3 * v + 1], b.wpos[3 * v + 2], __longlong_as_double((long long)v));
+    }
+}
+
+// nei_off from nei_cnt, the largest count in status[1]
+__global__ void __launch_bounds__(kSmallThreads) k_small_offsets(Batch b) {
+    __shared__ int wsum[32];
+    __shared__ int top;
+    const int tid = threadIdx.x;
+    constexpr int kPer = kSmallAtoms / kSmallThreads;
+    if (tid == 0) top = 0;
+    int v[kPer], sum = 0, most = 0, total;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int i = tid * kPer + u;
+        v[u] = i < b.natoms ? b.nei_cnt[i] : 0;
+        sum += v[u];
+        most = max(most, v[u]);
+    }
+    int at = block_exclusive(sum, wsum, &total);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((tid & 31) == 0) atomicMax(&top, most);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int i = tid * kPer + u;
+        if (i < b.natoms) b.nei_off[i] = at;
+        at += v[u];
+    }
+    __syncthreads();
+    if (tid == 0) {
+        b.nei_off[b.natoms] = total;
+        b.status[1] = top;
+    }
+}
+
 // Padded rows -> CSR lists (plans, eager calls after the first), one warp
 // per atom, lanes over its entries; with the slab table it also writes the
 // reverse index: the entry (j -> i, -S) of (i -> j, S) found in slab s lies
@@ -577,6 +826,21 @@ int launch_scan(int* data, int n, int* tmp, int* total_unused, cudaStream_t s) {
     return launch_scan_from(data, data, n, tmp, s);
 }
 
+// Largest number of cells per atom for the warp-per-cell search: beyond it
+// (plans of molecules, whose cells are reserved for the largest grid) most
+// warps would find an empty cell.
+constexpr int kCellsPerAtom = 4;
+// Smallest batch for it: one cell's chain is longer than one atom's, which
+// counts while the GPU is not full.  List stages with a warp per atom (a
+// thread per atom from 131,072 atoms) / a warp per cell, in us: 42 / 59 at 768
+// atoms, 125 / 116 at 18,000, 355 / 290 at 71,000, 723 / 637 at 191,000.
+constexpr int kCellListAtoms = 12288;
+
+// Batches whose list stages run in one block each: up to kSmallAtoms atoms the
+// chain of launches costs more than a single SM's work (768 atoms: cell stage
+// 18 us in five launches and two clears, 7 in one).
+static bool small_batch(const Batch& b) { return b.natoms <= kSmallAtoms && b.ncells < kSmallCells; }
+
 int launch_neighbour_build_a(const Batch& b, const DevModel& m, cudaStream_t s, bool sid_valid) {
     int L = 0;
     const int gA = (b.natoms + kThreads - 1) / kThreads;
@@ -584,22 +848,30 @@ int launch_neighbour_build_a(const Batch& b, const DevModel& m, cudaStream_t s, 
         k_atom_struct<<<b.nstruct, 128, 0, s>>>(b.info, b.nstruct, b.sid);
         ++L;
     }
-    cudaMemsetAsync(b.cell_cnt, 0, sizeof(int) * (b.ncells + 1), s);
-    k_wrap_bin<<<gA, kThreads, 0, s>>>(b, m);
-    ++L;
-    L += launch_scan_from(b.cell_cnt, b.cell_start, b.ncells, b.scan_tmp, s);
-    cudaMemsetAsync(b.cell_cnt, 0, sizeof(int) * (b.ncells + 1), s);
-    k_fill_cells<<<gA, kThreads, 0, s>>>(b, b.cell_cnt);
-    ++L;
-    k_sort_cells<<<(unsigned)((32LL * b.ncells + kThreads - 1) / kThreads), kThreads, 0, s>>>(b);
-    ++L;
-    if (b.posc) {
-        k_cell_positions<<<gA, kThreads, 0, s>>>(b);
+    const bool small = small_batch(b);
+    if (small) {
+        k_small_cells<<<1, kSmallThreads, 0, s>>>(b, m);
         ++L;
+    } else {
+        cudaMemsetAsync(b.cell_cnt, 0, sizeof(int) * (b.ncells + 1), s);
+        k_wrap_bin<<<gA, kThreads, 0, s>>>(b, m);
+        ++L;
+        L += launch_scan_from(b.cell_cnt, b.cell_start, b.ncells, b.scan_tmp, s);
+        cudaMemsetAsync(b.cell_cnt, 0, sizeof(int) * (b.ncells + 1), s);
+        k_fill_cells<<<gA, kThreads, 0, s>>>(b, b.cell_cnt);
+        ++L;
+        k_sort_cells<<<(unsigned)((32LL * b.ncells + kThreads - 1) / kThreads), kThreads, 0, s>>>(b);
+        ++L;
+        if (b.posc) {
+            k_cell_positions<<<gA, kThreads, 0, s>>>(b);
+            ++L;
+        }
     }
     const unsigned gW = (unsigned)((32LL * b.natoms + kThreads - 1) / kThreads);
     if (b.pad_cap > 0) {  // plans: one search pass into padded rows
-        if (warp_lists(b))
+        if (b.nei_warp == 0 && b.posc && b.natoms >= kCellListAtoms && b.ncells <= kCellsPerAtom * (long long)b.natoms)
+            k_neighbours_cell<<<(b.ncells + kCellWarps - 1) / kCellWarps, 32 * kCellWarps, 0, s>>>(b, m);
+        else if (warp_lists(b))
             k_neighbours_warp<2><<<gW, kThreads, 0, s>>>(b, m);
         else
             k_neighbours<2><<<gA, kThreads, 0, s>>>(b, m);
@@ -609,6 +881,10 @@ int launch_neighbour_build_a(const Batch& b, const DevModel& m, cudaStream_t s, 
         k_neighbours<0><<<gA, kThreads, 0, s>>>(b, m);
     }
     ++L;
+    if (small) {
+        k_small_offsets<<<1, kSmallThreads, 0, s>>>(b);
+        return L + 1;
+    }
     L += launch_scan_from(b.nei_cnt, b.nei_off, b.natoms, b.scan_tmp, s);
     // status[1] = max count
     cudaMemsetAsync(b.status + 1, 0, sizeof(int), s);
@@ -751,6 +1027,22 @@ __global__ void k_caps_clear(Batch b) {
     if (i <= b.natoms && b.status[3]) b.nei_off[i] = 0;
 }
 
+// both for a small batch
+__global__ void __launch_bounds__(kSmallThreads) k_caps_small(Batch b, long long e_cap, int m_cap) {
+    __shared__ int bad;
+    if (threadIdx.x == 0) {
+        const int total = b.nei_off[b.natoms];
+        bad = total < 0 || (long long)total > e_cap || b.status[1] > m_cap;
+        if (bad) {
+            atomicOr(&b.status[0], 32);
+            b.status[3] = 1;
+        }
+    }
+    __syncthreads();
+    if (bad)
+        for (int i = threadIdx.x; i <= b.natoms; i += kSmallThreads) b.nei_off[i] = 0;
+}
+
 // Device copies of the host set-up arithmetic (struct_setup, n_cells and inv3
 // in capi.cu) with every operation rounded on its own (no contraction), so the
 // device-built box of a molecule equals the host-built one bit for bit.
@@ -883,6 +1175,10 @@ __global__ void k_molecule_boxes(Batch b, double rc) {
 }  // namespace
 
 int launch_capacity_guard(const Batch& b, long long e_cap, int m_cap, cudaStream_t s) {
+    if (b.natoms <= kSmallAtoms) {
+        k_caps_small<<<1, kSmallThreads, 0, s>>>(b, e_cap, m_cap);
+        return 1;
+    }
     k_caps_check<<<1, 32, 0, s>>>(b, e_cap, m_cap);
     k_caps_clear<<<(b.natoms + 1 + kThreads - 1) / kThreads, kThreads, 0, s>>>(b);
     return 2;
