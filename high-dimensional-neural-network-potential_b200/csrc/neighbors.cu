@@ -835,6 +835,9 @@ constexpr int kCellsPerAtom = 4;
 // thread per atom from 131,072 atoms) / a warp per cell, in us: 42 / 59 at 768
 // atoms, 125 / 116 at 18,000, 355 / 290 at 71,000, 723 / 637 at 191,000.
 constexpr int kCellListAtoms = 12288;
+// Largest one: from here a thread per atom keeps the GPU full (1.93 ms of the
+// 758,676-atom step, against about 2.6).
+constexpr int kCellListMost = 262144;
 
 // Batches whose list stages run in one block each: up to kSmallAtoms atoms the
 // chain of launches costs more than a single SM's work (768 atoms: cell stage
@@ -869,7 +872,8 @@ int launch_neighbour_build_a(const Batch& b, const DevModel& m, cudaStream_t s, 
     }
     const unsigned gW = (unsigned)((32LL * b.natoms + kThreads - 1) / kThreads);
     if (b.pad_cap > 0) {  // plans: one search pass into padded rows
-        if (b.nei_warp == 0 && b.posc && b.natoms >= kCellListAtoms && b.ncells <= kCellsPerAtom * (long long)b.natoms)
+        if (b.nei_warp == 0 && b.posc && b.natoms >= kCellListAtoms && b.natoms < kCellListMost &&
+            b.ncells <= kCellsPerAtom * (long long)b.natoms)
             k_neighbours_cell<<<(b.ncells + kCellWarps - 1) / kCellWarps, 32 * kCellWarps, 0, s>>>(b, m);
         else if (warp_lists(b))
             k_neighbours_warp<2><<<gW, kThreads, 0, s>>>(b, m);
