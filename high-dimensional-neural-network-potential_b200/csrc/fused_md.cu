@@ -25,6 +25,7 @@
 #include <atomic>
 
 #include "engine.h"
+#include "fastmath.cuh"
 #include "mlp_tile.cuh"
 #include "symfn_generic.cuh"
 
@@ -344,10 +345,10 @@ size_t small_md_layout(const DevModel& m, int N, FusedArgs* a) {
 // entry, an angular pair (j, k) of one centre, or one (atom, symmetry
 // function) -- and every sum is taken in a fixed order by one thread
 // (deterministic):
-//   entries: geometry, cutoff and the radial exponentials of the entry's
-//            (centre, neighbour element) group;
+//   entries: geometry and cutoff; then, per function of its (centre,
+//            neighbour element) group, the radial exponential;
 //   pairs:   the angular geometry of (j, k) (oriented like the element pair
-//            block: j of its first element) and, per function of the block,
+//            block: j of its first element); then, per function of the block,
 //            exp(-eta (rij^2 + rik^2 + rjk^2)) and (1 + lambda cos)^(zeta-1);
 //   values:  G of one (atom, function) from the entry / pair terms;
 //   network: one (atom, neuron) per thread, layer by layer; stores
@@ -357,6 +358,8 @@ size_t small_md_layout(const DevModel& m, int N, FusedArgs* a) {
 //   entry gradients: radial part + the pair parts of one entry.
 // The formulas are those of the generic per-atom routines (symfn_generic.cuh,
 // after symmetryFunctions.f90:129-297 of the reference).
+
+constexpr int kTinyThreads = 512;
 
 enum TSlot {
     tPos, tMom, tF, tFp, tMass, tAtE, tG, tW, tEG, tERC, tGent, tPS, tPE, tPT, tPG, tMlp,
@@ -409,7 +412,25 @@ __device__ __forceinline__ int owner_of(const int* off, int n, int x) {
     return lo;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a) {
+// cutoff of symfn_generic.cuh in the branch-free functions of fastmath.cuh
+__device__ __forceinline__ void tiny_cutoff(double r, double ir, double irc, double rc, double& fc, double& dfc) {
+    fc = dfc = 0.0;
+    if (r < rc) {
+        const double t = tanh01(1.0 - r * irc), tt = t * t;
+        fc = tt * t;
+        dfc = -3.0 * irc * ir * (tt - tt * tt);
+    }
+}
+
+// Latency-bound: one block, a dozen stages of a few microseconds' chains.  So
+// the exponentials and powers, the longest links, are items of their own
+// ((entry, function) and (pair, function)) spread over all threads, and the
+// transcendental functions and divisions are the short forms of fastmath.cuh;
+// every warp scans the list offsets for itself instead of waiting for one, and
+// a value's sum over pairs has no branch.  Per step of the 8-atom example 15.7
+// us before (a thread's functions one after the other, library functions, 256
+// threads), 14.7 now.
+__global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_md(DevModel m, TinyArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
     const int N = a.natoms, n3 = 3 * N, nel = m.nel, nblk = m.nblk, nsf = m.nsf_max;
@@ -525,51 +546,60 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
             if (lane == 0) mask[i] = mk;
         }
         __syncthreads();
-        // entry and pair offsets (warp 0, two atoms per lane)
-        if (w == 0) {
+        // entries: index order, reverse entry by popcount, geometry, radial exponentials
+        // (entry and pair offsets: every warp scans the counts for itself, two
+        // atoms per lane, and warp 0 writes them down)
+        int offe;  // first entry of atom 2 lane, the next atom's behind its own
+        int cnt0;
+        {
             const int i0 = 2 * lane, i1 = 2 * lane + 1;
             const int c0 = i0 < N ? __popcll(mask[i0]) : 0, c1 = i1 < N ? __popcll(mask[i1]) : 0;
             const int q0 = c0 * (c0 - 1) / 2, q1 = c1 * (c1 - 1) / 2;
-            int ie = c0 + c1, ip = q0 + q1;
-            for (int d = 1; d < 32; d <<= 1) {
-                const int te = __shfl_up_sync(0xffffffffu, ie, d), tp = __shfl_up_sync(0xffffffffu, ip, d);
-                if (lane >= d) {
-                    ie += te;
-                    ip += tp;
+            long long sum = (long long)(c0 + c1) | ((long long)(q0 + q1) << 32);
+            for (int d = 1; 2 * d < N + 2 && d < 32; d <<= 1) {
+                const long long o = __shfl_up_sync(0xffffffffu, sum, d);
+                if (lane >= d) sum += o;
+            }
+            const int xe = (int)(sum & 0xffffffff) - c0 - c1, xp = (int)(sum >> 32) - q0 - q1;
+            offe = xe;
+            cnt0 = c0;
+            if (w == 0) {
+                if (i0 <= N) {
+                    off[i0] = xe;
+                    poff[i0] = xp;
+                }
+                if (i1 <= N) {
+                    off[i1] = xe + c0;
+                    poff[i1] = xp + q0;
+                }
+                if (lane == 31 && N == 64) {
+                    off[N] = xe + c0 + c1;
+                    poff[N] = xp + q0 + q1;
                 }
             }
-            const int xe = ie - c0 - c1, xp = ip - q0 - q1;
-            if (i0 < N) {
-                off[i0] = xe;
-                poff[i0] = xp;
-            }
-            if (i1 < N) {
-                off[i1] = xe + c0;
-                poff[i1] = xp + q0;
-            }
-            if (lane == 31) {
-                off[N] = ie;
-                poff[N] = ip;
-            }
         }
-        __syncthreads();
-        // entries: index order, reverse entry by popcount, geometry, radial exponentials
+        // first entry of atom j
+        auto first_entry = [&](int j) {
+            const int e = __shfl_sync(0xffffffffu, offe, j >> 1), c = __shfl_sync(0xffffffffu, cnt0, j >> 1);
+            return (j & 1) ? e + c : e;
+        };
         for (int i = w; i < N; i += nw) {
             const unsigned long long mi = mask[i];
-            const int o = off[i], c = elem[i];
-            const double rc = m.rc[c];
+            const int o = first_entry(i), c = elem[i];
+            const double rc = m.rc[c], irc = 1.0 / rc;
             const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
             for (int cc = 0; cc < N; cc += 32) {
                 const int j = cc + lane;
+                const int oj = first_entry(min(j, 63));
                 if (j < N && ((mi >> j) & 1ull)) {
                     const int e = o + __popcll(mi & ((1ull << j) - 1ull));
                     nj[e] = j;
                     own[e] = i;
-                    rev[e] = off[j] + __popcll(mask[j] & ((1ull << i) - 1ull));
+                    rev[e] = oj + __popcll(mask[j] & ((1ull << i) - 1ull));
                     const double dx = xi - pos[3 * j], dy = yi - pos[3 * j + 1], dz = zi - pos[3 * j + 2];
-                    const double r = sqrt(dx * dx + dy * dy + dz * dz);
-                    double fc, dfc;
-                    cutoff(r, rc, fc, dfc);
+                    double r, ir, fc, dfc;
+                    sqrt_rsqrt(dx * dx + dy * dy + dz * dz, r, ir);
+                    tiny_cutoff(r, ir, irc, rc, fc, dfc);
                     double* ge = eg + 6 * e;
                     ge[0] = dx;
                     ge[1] = dy;
@@ -577,16 +607,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
                     ge[3] = r;
                     ge[4] = fc;
                     ge[5] = dfc;
-                    const int el = elem[j], f0 = m.g2_off[c * nel + el], f1 = m.g2_off[c * nel + el + 1];
-                    for (int f = f0; f < f1; ++f) {
-                        const SF2 q = m.g2[f];
-                        const double x = r - q.rs;
-                        erc[(size_t)e * g2w + (f - f0)] = exp(-q.eta * x * x);
-                    }
                 }
             }
         }
         __syncthreads();
+        // radial exponentials, one (entry, function) per thread, from the last
+        // thread down (the first ones have the pairs)
+        const int nent = off[N];
+        for (int x = nt - 1 - tid; x < nent * m.g2el_max; x += nt) {
+            const int e = x / m.g2el_max, f = x - e * m.g2el_max;
+            const int g = elem[own[e]] * nel + elem[nj[e]], f0 = m.g2_off[g];
+            if (f < m.g2_off[g + 1] - f0) {
+                const SF2 q = m.g2[f0 + f];
+                const double d = eg[6 * e + 3] - q.rs;
+                erc[(size_t)e * g2w + f] = exp_clamped(-q.eta * d * d);
+            }
+        }
         // angular pairs
         const int npair = poff[N];
         for (int P = tid; P < npair; P += nt) {
@@ -608,24 +644,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
             const double rjk2 = cx * cx + cy * cy + cz * cz;
             if (!(rjk2 < mrc * mrc)) continue;
             const double rj = aj[3], rk = ak[3];
-            const double rjk = sqrt(rjk2);
-            double fjk, dfjk;
-            cutoff(rjk, mrc, fjk, dfjk);
+            double rjk, irjk, fjk, dfjk;
+            sqrt_rsqrt(rjk2, rjk, irjk);
+            tiny_cutoff(rjk, irjk, 1.0 / mrc, mrc, fjk, dfjk);
             const double t1 = -1.0 / (rj * rk);
             const double cth = 0.5 * (rjk * rjk - rj * rj - rk * rk) * t1;
             const double fcp = aj[4] * ak[4] * fjk;
-            const double rsum = rj * rj + rk * rk + rjk * rjk;
-            double last_eta = -1.0, ex = 0.0;
-            for (int u = 0; u < ge - gb; ++u) {
-                const SF4 f = m.g4[gb + u];
-                if (f.eta != last_eta) {
-                    ex = exp(-f.eta * rsum);
-                    last_eta = f.eta;
-                }
-                const double base = 1.0 + f.lambda * cth;
-                pe[(size_t)P * g4w + u] = ex;
-                pt[(size_t)P * g4w + u] = f.izeta >= 0 ? ipow(base, f.izeta - 1) : pow(base, f.zeta - 1.0);
-            }
             double* s = ps + 5 * (size_t)P;
             s[0] = fjk;
             s[1] = dfjk;
@@ -634,6 +658,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
             s[4] = fcp;
             pblk[P] = t | (swap ? 256 : 0);
             pjk[P] = j | (k << 16);
+        }
+        __syncthreads();
+        // per function of the pair's block: exponential and power, one (pair,
+        // function) per thread
+        for (int x = tid; x < npair * g4w; x += nt) {
+            const int P = x / g4w, u = x - P * g4w, pb = pblk[P];
+            if (pb < 0) continue;
+            const int j = pjk[P] & 0xffff, k = pjk[P] >> 16, g = elem[own[j]] * nblk + (pb & 255);
+            if (u >= m.g4_off[g + 1] - m.g4_off[g]) continue;
+            const SF4 f = m.g4[m.g4_off[g] + u];
+            const double* aj = eg + 6 * j;
+            const double* ak = eg + 6 * k;
+            const double cx = ak[0] - aj[0], cy = ak[1] - aj[1], cz = ak[2] - aj[2];
+            const double rsum = aj[3] * aj[3] + ak[3] * ak[3] + (cx * cx + cy * cy + cz * cz);
+            const double base = 1.0 + f.lambda * ps[5 * (size_t)P + 3];
+            pe[x] = exp_clamped(-f.eta * rsum);
+            pt[x] = f.izeta >= 0 ? ipow(base, f.izeta - 1) : pow(base, f.zeta - 1.0);
         }
         __syncthreads();
         // symmetry-function values, one (atom, function) per thread
@@ -652,19 +693,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
             } else if (u < n2 + n4) {
                 const int g = a0 + u - n2, t = recblk[g], col = g - m.g4_off[c * nblk + t];
                 const SF4 f = m.g4[g];
-                for (int P = poff[i]; P < poff[i + 1]; ++P) {
+                // without a branch per pair (the lanes' functions belong to
+                // different blocks, so nearly every pair is some lane's)
+                const int P1 = poff[i + 1];
+#pragma unroll 4
+                for (int P = poff[i]; P < P1; ++P) {
                     const int pb = pblk[P];
-                    if (pb < 0 || (pb & 255) != t) continue;
-                    const double* s = ps + 5 * (size_t)P;
+                    const double* s = ps + 5 * P;
                     const double base = 1.0 + f.lambda * s[3];
-                    acc += f.pf * (pt[(size_t)P * g4w + col] * base) * pe[(size_t)P * g4w + col] * s[4];
+                    const double v = f.pf * (pt[P * g4w + col] * base) * pe[P * g4w + col] * s[4];
+                    acc += (pb >= 0 && (pb & 255) == t) ? v : 0.0;
                 }
                 sf = f.sf;
             } else {
                 continue;
             }
             const size_t k = (size_t)c * nsf + sf;
-            G[(size_t)i * nsf + sf] = (acc - m.smean[k]) / m.swidth[k];
+            G[(size_t)i * nsf + sf] = (acc - m.smean[k]) * m.sinvw[k];
         }
         __syncthreads();
         // networks: one (atom, neuron) per thread and layer; activations in mlp
@@ -716,7 +761,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
                     double s = 0.0;
                     for (int o = 0; o < wout; ++o) s += da[o] * Wm[(size_t)o * wi + k];
                     if (l == 0)
-                        Wt[(size_t)i * nsf + k] = s / m.swidth[(size_t)e * nsf + k];
+                        Wt[(size_t)i * nsf + k] = s * m.sinvw[(size_t)e * nsf + k];
                     else
                         d1[x] = s * act_d(m.act[l - 1], cp[x], yp[x]);
                 }
@@ -740,8 +785,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
             const double rj = aj[3], rk = ak[3], fj = aj[4], fk = ak[4], dfj = aj[5], dfk = ak[5];
             const double cx = akx - ajx, cy = aky - ajy, cz = akz - ajz;
             const double fjk = s[0], dfjk = s[1], t1 = s[2], cth = s[3], fcp = s[4];
-            const double dot = ajx * akx + ajy * aky + ajz * akz;
-            const double cj = dot / (rj * rj * rj * rk), ck = dot / (rk * rk * rk * rj);
+            // (r_ij . r_ik) / (r_ij^3 r_ik) = cos / r_ij^2
+            const double cj = cth / (rj * rj), ck = cth / (rk * rk);
             double A = 0.0, B = 0.0, C = 0.0;
             for (int u = 0; u < ge - gb; ++u) {
                 const SF4 f = m.g4[gb + u];
@@ -763,18 +808,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiny_md(DevModel m, TinyArgs a)
         }
         __syncthreads();
         // entry gradients: radial part, then the pair parts in pair order
-        const int nent = off[N];
         for (int e = tid; e < nent; e += nt) {
             const int i = own[e], c = elem[i], p = e - off[i], M = off[i + 1] - off[i];
             const int el = elem[nj[e]], f0 = m.g2_off[c * nel + el], f1 = m.g2_off[c * nel + el + 1];
             const double* ge = eg + 6 * e;
             const double r = ge[3], fc = ge[4], dfc = ge[5];
+            const double ir = 1.0 / r;
             double coef = 0.0;
             for (int f = f0; f < f1; ++f) {
                 const SF2 q = m.g2[f];
                 const double x = r - q.rs;
                 const double ex = erc[(size_t)e * g2w + (f - f0)];
-                coef += Wt[(size_t)i * nsf + q.sf] * (-ex * dfc + 2.0 * q.eta * x / r * ex * fc);
+                coef += Wt[(size_t)i * nsf + q.sf] * (-ex * dfc + 2.0 * q.eta * x * ir * ex * fc);
             }
             double gx = coef * ge[0], gy = coef * ge[1], gz = coef * ge[2];
             for (int qq = 0; qq < M; ++qq) {
@@ -915,7 +960,7 @@ int launch_small_resident(const DevModel& m, int natoms, ResidentBox* box, cudaS
     ta.eval_only = 1;
     ta.box = box;
     cudaFuncSetAttribute(k_tiny_md, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
-    k_tiny_md<<<1, kThreads, tsm, s>>>(m, ta);
+    k_tiny_md<<<1, kTinyThreads, tsm, s>>>(m, ta);
     return 1;
 }
 
@@ -957,7 +1002,7 @@ int launch_small_md(const Batch& b, const DevModel& m, const SmallMdArgs& x, cud
                 }
             }
         }
-        k_tiny_md<<<1, kThreads, tsm, s>>>(m, ta);
+        k_tiny_md<<<1, kTinyThreads, tsm, s>>>(m, ta);
         return 1;
     }
     FusedArgs a{};
