@@ -198,6 +198,8 @@ struct hdnnp_ctx {
     DevBuf<double> cm_acc, cm_E, cm_std;                  // committee: dE/dG sum, member energies, std
     DevBuf<unsigned> pairs;                               // contributing-pair lists (fast kernels)
     DevBuf<int> npairs, wide;
+    cudaStream_t side = nullptr;                          // SF launches of atoms with many neighbours
+    cudaEvent_t fork = nullptr, join = nullptr;
     DevBuf<int> cnei_cnt, cnei_off, cnei_j, cnei_s, cnei_rev, cnei_map;  // compacted Verlet-skin lists
     DevBuf<int> pad;                                      // padded neighbour rows (int2 pairs)
     DevBuf<double4> posc;                                 // cell-ordered wrapped positions
@@ -266,6 +268,9 @@ struct hdnnp_ctx {
         if (rs_stream) cudaStreamDestroy(rs_stream);
         if (se_dev) cudaFree(se_dev);
         if (se_host) cudaFreeHost(se_host);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -830,9 +835,15 @@ int run_pipeline(hdnnp_ctx* c, int nstruct, int natoms, const int32_t* Zd, const
     mixed = c->precision == HDNNP_PREC_MIXED && fast;
     if (fast) {
         if ((r = c->pairs.ensure(N * (size_t)kPairCap)) || (r = c->npairs.ensure(N)) ||
-            (r = c->wide.ensure(N + 2)))
+            (r = c->wide.ensure(N + 1)))
             return r;
+        if (!c->side) CUDA_TRY(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+        for (auto* e : {&c->fork, &c->join})
+            if (!*e) CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         b.wide = c->wide.p;
+        b.side = c->side;
+        b.fork = c->fork;
+        b.join = c->join;
         b.pairs = c->pairs.p;
         b.npairs = c->npairs.p;
         b.pcap = kPairCap;

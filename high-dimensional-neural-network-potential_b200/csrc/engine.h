@@ -193,10 +193,12 @@ struct Batch {
     unsigned* pairs;          // [natoms * pcap]
     int* npairs;              // [natoms]
     int pcap;
-    // Atoms with more neighbours than the first launch of a fast pass takes:
-    // [0] and [1] their number in the value and the gradient pass, then the
-    // list (each pass its own, one after the other).
-    int* wide;                // [natoms + 2]
+    // Atoms with more neighbours than the main launch of a fast pass takes:
+    // their number, then the list.  They run on the context's side stream,
+    // forked from and joined to the evaluation's stream by the two events.
+    int* wide;                // [natoms + 1]
+    cudaStream_t side;
+    cudaEvent_t fork, join;
     // Launch shape of the fast symmetry-function kernels (0: defaults): the
     // neighbour count splitting the two launches (-1: one launch) and the
     // persistent grid in blocks per SM.  Set by the plans' autotuner.

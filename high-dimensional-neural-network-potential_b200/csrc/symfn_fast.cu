@@ -32,17 +32,18 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarps = 4;
 // parts of a pass: one launch for all atoms, or one for those with few
-// neighbours, which lists the others, and one for the listed
+// neighbours and one for the listed others
 constexpr int kPartAll = 0, kPartFirst = 1, kPartWide = 2;
 // Resident blocks per SM that the kernels are compiled for (registers) and
 // the default split of a pass is sized for (shared memory): value pass 5 FP64
 // (96 registers) and 6 FP32; gradient pass 4 FP64 (122 registers, no spills;
 // at 5 its four accumulator copies leave 44 neighbours and the pass takes
-// 5.4 ms instead of 3.6 on 1024 structures) and 7 FP32.
+// 5.4 ms instead of 3.6 on 1024 structures) and 6 FP32 (2.31 ms, 2.44 at 7
+// with spills).
 template <typename T>
 constexpr int kBlocksV = sizeof(T) == 4 ? 6 : 5;
 template <typename T>
-constexpr int kBlocksG = sizeof(T) == 4 ? 7 : 4;
+constexpr int kBlocksG = sizeof(T) == 4 ? 6 : 4;
 
 template <typename T>
 struct alignas(4 * sizeof(T)) V4 {
@@ -762,16 +763,15 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, 
     unsigned long long st_ent = 0, st_cand = 0, st_pairs = 0, st_g2 = 0;
     const int total_atoms = part == kPartWide ? b.wide[0] : b.natoms;
     for (int q = blockIdx.x * nw + wib; q < total_atoms; q += gridDim.x * nw) {
-        const int i = part == kPartWide ? b.wide[2 + q] : q;
+        const int i = part == kPartWide ? b.wide[1 + q] : q;
         const int c = b.elem[i];
         if (c < 0) continue;
         const int M = b.nei_off[i + 1] - b.nei_off[i];
-        // more neighbours than this launch's shared memory takes: to the list
-        // of the launch that follows (see run_form)
+        // more neighbours than this launch's shared memory takes: listed for
+        // the launch beside it (see run_form)
         if (M > mm) {
             if (lane == 0) {
-                if (part == kPartFirst) b.wide[2 + atomicAdd(&b.wide[0], 1)] = i;
-                else atomicOr(&b.status[0], 4);
+                if (part != kPartFirst) atomicOr(&b.status[0], 4);
             }
             continue;
         }
@@ -1206,18 +1206,17 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksG<T>) k_sfg_fast(Batch b, 
     const int nel = m.nel;
     const T* dEdG = Buf<T>::dEdG(b);
     const int ne = n_eta<S>(m);
-    const int total_atoms = part == kPartWide ? b.wide[1] : b.natoms;
+    const int total_atoms = part == kPartWide ? b.wide[0] : b.natoms;
     for (int q = blockIdx.x * nw + wib; q < total_atoms; q += gridDim.x * nw) {
-        const int i = part == kPartWide ? b.wide[2 + q] : q;
+        const int i = part == kPartWide ? b.wide[1 + q] : q;
         const int c = b.elem[i];
         if (c < 0) continue;
         const int M = b.nei_off[i + 1] - b.nei_off[i];
-        // more neighbours than this launch's shared memory takes: to the list
-        // of the launch that follows (see run_form)
+        // more neighbours than this launch's shared memory takes: listed for
+        // the launch beside it (see run_form)
         if (M > mm) {
             if (lane == 0) {
-                if (part == kPartFirst) b.wide[2 + atomicAdd(&b.wide[1], 1)] = i;
-                else atomicOr(&b.status[0], 4);
+                if (part != kPartFirst) atomicOr(&b.status[0], 4);
             }
             continue;
         }
@@ -1361,6 +1360,19 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksG<T>) k_sfg_fast(Batch b, 
     }
 }
 
+// atoms with more than mm neighbours: their number in b.wide[0], then the list
+// (in no particular order; every atom's result is its own)
+__global__ void k_list_wide(Batch b, int mm) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const bool w = i < b.natoms && b.nei_off[i + 1] - b.nei_off[i] > mm;
+    const unsigned bal = __ballot_sync(kFull, w);
+    int base = 0;
+    if (lane == 0 && bal) base = atomicAdd(&b.wide[0], __popc(bal));
+    base = __shfl_sync(kFull, base, 0);
+    if (w) b.wide[1 + base + __popc(bal & lanemask_lt())] = i;
+}
+
 int nsm() { return device_sm_count(); }
 
 constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory of a block
@@ -1374,13 +1386,15 @@ void set_smem(K kernel, size_t smem) {
 
 // Shared memory per warp grows with the largest neighbour count of the
 // batch, and it sets how many warps an SM holds.  Atoms with at most `split`
-// neighbours run in a launch sized for that count, which lists the others;
-// those follow in a second launch sized for the batch maximum.  Each atom is
-// evaluated once, by the same code.  (A second launch that searched all atoms
-// for its own took 0.3 ms of a 1024-structure step, nearly all of it latency.)
+// neighbours run in a launch sized for that count; the others are listed and
+// run in a launch sized for the batch maximum, beside the first one on the
+// context's side stream (after it, the few listed atoms took 80 of the 440 us
+// of each pass for 96 structures, one atom's latency on a nearly idle GPU).
+// Each atom is evaluated once, by the same code.
 // The split and the persistent grid (blocks per SM) are the knobs of the
 // plans' autotuner (Batch::sf_split, Batch::sf_blocks_per_sm).
 constexpr int kBlocksPerSm = 32;
+constexpr int kWideBlocksPerSm = 2;  // of the launch for the listed atoms
 
 template <typename T, class S, bool kB>
 int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
@@ -1400,30 +1414,36 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
         if ((long long)b.natoms <= (long long)nsm() * fit * kWarps) split = mfull;
     }
     int L = 0;
-    auto go = [&](int mm, int part) {
+    auto go = [&](int mm, int part, cudaStream_t on) {
         // four warps a block, fewer where so many neighbours do not fit
         int nw = kWarps;
         while (nw > 1 && warp_bytes(mm) * nw > kSmemMax) nw >>= 1;
         const size_t smem = warp_bytes(mm) * nw;
         int blocks = (b.natoms + nw - 1) / nw;
-        const int cap = nsm() * per_sm;
+        const int cap = nsm() * (part == kPartWide ? kWideBlocksPerSm : per_sm);
         if (blocks > cap) blocks = cap;
         if (blocks < 1) blocks = 1;
         if (grad) {
             set_smem(k_sfg_fast<T, S, kB>, smem);
-            k_sfg_fast<T, S, kB><<<blocks, 32 * nw, smem, st>>>(b, m, mm, part);
+            k_sfg_fast<T, S, kB><<<blocks, 32 * nw, smem, on>>>(b, m, mm, part);
         } else {
             set_smem(k_sfv_fast<T, S, kB>, smem);
-            k_sfv_fast<T, S, kB><<<blocks, 32 * nw, smem, st>>>(b, m, mm, part);
+            k_sfv_fast<T, S, kB><<<blocks, 32 * nw, smem, on>>>(b, m, mm, part);
         }
         ++L;
     };
     if (mfull > split) {
-        cudaMemsetAsync(b.wide + (grad ? 1 : 0), 0, sizeof(int), st);
-        go(split, kPartFirst);
-        go(mfull, kPartWide);
+        cudaMemsetAsync(b.wide, 0, sizeof(int), st);
+        k_list_wide<<<(b.natoms + 255) / 256, 256, 0, st>>>(b, split);
+        ++L;
+        cudaEventRecord(b.fork, st);
+        cudaStreamWaitEvent(b.side, b.fork, 0);
+        go(mfull, kPartWide, b.side);
+        go(split, kPartFirst, st);
+        cudaEventRecord(b.join, b.side);
+        cudaStreamWaitEvent(st, b.join, 0);
     } else {
-        go(mfull, kPartAll);
+        go(mfull, kPartAll, st);
     }
     return L;
 }
