@@ -218,8 +218,8 @@ def measured_peaks(torch):
 # reference's per-function loops; the roofline is therefore stated with the
 # algorithmic count below and the executed count beside it.
 FLOPS_EXECUTED = {
-    "sf_values": {"entries": 30, "pairs": 88, "g2_terms": 6},
-    "sf_gradients": {"entries": 57, "pairs": 263, "g2_terms": 13},
+    "sf_values": {"entries": 30, "pairs": 71, "g2_terms": 6},
+    "sf_gradients": {"entries": 57, "pairs": 178, "g2_terms": 13},
 }
 
 # Algorithmic operations per work unit of the reference's path (one value +

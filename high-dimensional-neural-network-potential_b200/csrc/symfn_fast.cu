@@ -125,8 +125,13 @@ struct FSmem {
 __host__ __device__ inline int mask_words(int mm) { return (mm + 31) / 32 * 32; }
 // pairs the value pass lists at a time: a row (one neighbour's pairs) and a
 // chunk's remainder always fit
-constexpr int kListCap = 160;
-__host__ __device__ inline int list_cap(int mm) { return mm + 32 > kListCap ? mm + 32 : kListCap; }
+// (1024 structures, value pass in ms: FP64 3.50, 3.43, 3.47 at 160, 192, 224;
+// FP32 2.86, 2.71, 2.93 at 160, 320, 640: fewer refills against fewer
+// neighbours per warp)
+template <typename T>
+constexpr int kListCap = sizeof(T) == 4 ? 320 : 192;
+template <typename T>
+__host__ __device__ inline int list_cap(int mm) { return mm + 32 > kListCap<T> ? mm + 32 : kListCap<T>; }
 
 template <typename T, class S>
 __host__ __device__ inline size_t fast_warp_bytes(int mm, int nel, int g2max, int nblk, bool grad) {
@@ -134,7 +139,7 @@ __host__ __device__ inline size_t fast_warp_bytes(int mm, int nel, int g2max, in
     if (grad) b += kCopies * 3 * a16(sizeof(T) * mm) + a16(sizeof(int) * mm) + a16(sizeof(T) * g2max) + a16(sizeof(T) * nblk * kWp<S>);
     else b += (sizeof(T) == 4 ? a16(sizeof(double4) * mm) : 0) + a16(2 * sizeof(T) * mm) +
               (kTRows<S> + 8) * kTs * sizeof(T) + a16(sizeof(unsigned) * mask_words(mm)) + a16(nel * nel);
-    b += a16(sizeof(unsigned) * (grad ? 64 : list_cap(mm))) + 3 * a16(sizeof(int) * kMaxEl) + a16(sizeof(int) * (kMaxEl + 1));
+    b += a16(sizeof(unsigned) * (grad ? 64 : list_cap<T>(mm))) + 3 * a16(sizeof(int) * kMaxEl) + a16(sizeof(int) * (kMaxEl + 1));
     return b;
 }
 
@@ -163,7 +168,7 @@ __device__ inline FSmem<T> fcarve(unsigned char* p, int mm, int nel, int g2max, 
         s.mask = (unsigned*)take(sizeof(unsigned) * mask_words(mm));
         s.tm = (unsigned char*)take(nel * nel);
     }
-    s.queue = (unsigned*)take(sizeof(unsigned) * (grad ? 64 : list_cap(mm)));
+    s.queue = (unsigned*)take(sizeof(unsigned) * (grad ? 64 : list_cap<T>(mm)));
     s.est = (int*)take(sizeof(int) * kMaxEl);
     s.cnt = (int*)take(sizeof(int) * kMaxEl);
     s.rst = (int*)take(sizeof(int) * (kMaxEl + 1));
@@ -756,7 +761,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, 
     // fragment rows and columns of this lane
     const T* ta = s.tb + (lane >> 2) * kTs + (lane & 3);
     const T* ya = s.yb + (lane >> 2) * kTs + (lane & 3);
-    const int cap = list_cap(mm);
+    const int cap = list_cap<T>(mm);
     for (int q = lane; q < 8 * kTs; q += 32) s.yb[q] = (T)0;
     __syncwarp();
     // work counters of this warp's atoms (profiling), added to b.stats once at the end
@@ -802,7 +807,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, 
                     const T r = live ? s.rf[2 * t] : (T)0;
                     const bool mine = live && rank >= x0 && rank < x0 + 8;
                     if (mine) s.yb[(rank - x0) * kTs + lane] = s.rf[2 * t + 1];
-#pragma unroll 2
+#pragma unroll (sizeof(T) == 8 ? 1 : 2)  // FP64: the smaller code is the faster one (3.49, 3.57, 3.69 ms at 1, 4, 8)
                     for (int f = 0; f < 8; ++f) {
                         T e = (T)0;
                         if (f < nf) {
@@ -862,9 +867,10 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, 
                     float kx = 1e18f, ky = 0.0f, kz = 0.0f;
                     if (k < Ms) cvec(s, k, kx, ky, kz);
                     unsigned mw = 0;
-                    for (int jj = 0; jj < nrow; jj += 4)
+                    // (rows up to a multiple of 8 lie inside the staging arrays)
+                    for (int jj = 0; jj < nrow; jj += 8)
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
+                        for (int u = 0; u < 8; ++u) {
                             float jx, jy, jz;
                             cvec(s, j0 + jj + u, jx, jy, jz);
                             const float ex = kx - jx, ey = ky - jy, ez = kz - jz;
@@ -1020,11 +1026,12 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, 
         }
         if (b.pairs && lane == 0) b.npairs[i] = n_pairs;
         if (b.stats) {
-            // radial terms: staged neighbours of each element x the centre's radial SFs for it
-            for (int el = 0; el < nel; ++el)
+            // per lane: radial terms (staged neighbours of an element x the
+            // centre's radial SFs for it) and candidates of an element pair
+            for (int el = lane; el < nel; el += 32)
                 st_g2 += (unsigned long long)s.cnt[el] *
                          (unsigned long long)(m.g2_off[c * nel + el + 1] - m.g2_off[c * nel + el]);
-            for (int t = 0; t < nblk; ++t)
+            for (int t = lane; t < nblk; t += 32)
                 if (m.g4_off[c * nblk + t + 1] > m.g4_off[c * nblk + t]) {
                     const int na = s.cnt[m.blk_a[t]], nb = s.cnt[m.blk_b[t]];
                     st_cand += m.blk_a[t] == m.blk_b[t] ? na * (na - 1) / 2 : na * nb;
@@ -1034,6 +1041,11 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, 
         }
         __syncwarp();
     }
+    if (b.stats)
+        for (int o = 16; o > 0; o >>= 1) {
+            st_cand += __shfl_xor_sync(kFull, st_cand, o);
+            st_g2 += __shfl_xor_sync(kFull, st_g2, o);
+        }
     if (b.stats && lane == 0 && st_ent) {
         atomicAdd(&b.stats[2], st_ent);
         atomicAdd(&b.stats[3], st_cand);
@@ -1404,8 +1416,8 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
     // allow still fit (1 KB of every block is the system's)
     const int resident = grad ? kBlocksG<T> : kBlocksV<T>;
     int fitting = 32;
-    while (fitting + 4 <= 1024 && (warp_bytes(fitting + 4) * kWarps + 1024) * resident <= 228 * 1024) fitting += 4;
-    int split = b.sf_split > 0 ? (b.sf_split + 3) / 4 * 4 : b.sf_split < 0 ? mfull : fitting;
+    while (fitting + 8 <= 1024 && (warp_bytes(fitting + 8) * kWarps + 1024) * resident <= 228 * 1024) fitting += 8;
+    int split = b.sf_split > 0 ? (b.sf_split + 7) / 8 * 8 : b.sf_split < 0 ? mfull : fitting;
     const int per_sm = b.sf_blocks_per_sm > 0 ? b.sf_blocks_per_sm : kBlocksPerSm;
     if (b.sf_split == 0 && mfull > split) {
         // a batch whose warps all fit on the GPU at the full size needs no

@@ -98,7 +98,8 @@ void hdnnp_ctx_free(hdnnp_ctx* c);
 int hdnnp_ctx_set_precision(hdnnp_ctx* c, int precision);
 
 /* Context options (for tests and tuning): "sf_split" (-1: one launch; 0:
- * default 64; n: atoms with more than n neighbours in a second launch) and
+ * default, the count whose shared memory keeps the kernels' blocks per SM
+ * resident; n: atoms with more than n neighbours in a second launch) and
  * "sf_blocks_per_sm" (0: default 32) shape the launches of the
  * lambda x zeta x eta kernels; "generic_sf" = 1 forces the
  * generic symmetry-function kernels (one parameter record per SF) instead of
