@@ -1707,14 +1707,17 @@ __global__ void k_math_check(int which, int n, const double* x, double* y) {
         case 0: r = exp_clamped(v); break;
         case 1: r = tanh01(v); break;
         case 2: sqrt_rsqrt(v, r, ir); break;
-        default: r = rsqrt_pos(v); break;
+        case 3: r = rsqrt_pos(v); break;
+        case 4: r = exp_small(v); break;
+        default: r = exp_neg(v); break;
     }
     y[i] = r;
 }
 }  // namespace
 
 extern "C" int hdnnp_debug_math(int which, int n, const double* x, double* y) {
-    if (which < 0 || which > 3) return fail(HDNNP_E_INPUT, "which must be 0 (exp), 1 (tanh), 2 (sqrt) or 3 (1/sqrt)");
+    if (which < 0 || which > 5)
+        return fail(HDNNP_E_INPUT, "which must be 0 (exp), 1 (tanh), 2 (sqrt), 3 (1/sqrt), 4 (exp on [-1.5, 0]) or 5 (exp on [-700, 0])");
     if (n < 0 || (n > 0 && (!x || !y))) return fail(HDNNP_E_INPUT, "null argument or negative count");
     if (n == 0) return HDNNP_OK;
     double* d = nullptr;

@@ -20,9 +20,14 @@
 //    libm (tests/test_fastmath.py emulates these operations on the host
 //    with exact fused multiply-adds, and checks the device functions, run
 //    through hdnnp_debug_math, against libm's exp, tanh and sqrt).
-//  * exp_small(x) for x in [-1.5, 0] and tanh01(u) for u in [0, 1]:
-//    polynomials interpolated at Chebyshev nodes (in 60 decimal digits, then
-//    rounded), two Horner chains each; no reduction, no reciprocal.
+//  * exp_neg(x): exp_clamped's operations for x in [-700, 0], without the
+//    clamp.  exp_small(x) for x in [-1.5, 0]: the same reduction (W. J. Cody,
+//    W. Waite, "Software Manual for the Elementary Functions", 1980) with ln 2
+//    in one double (at most two of them are taken off) and a polynomial
+//    interpolated at Chebyshev nodes on [-ln 2 / 2, ln 2 / 2].
+//  * tanh01(u) for u in [0, 1]: a polynomial interpolated at Chebyshev nodes;
+//    no reduction, no reciprocal.  (Both interpolants in 60 decimal digits,
+//    then rounded; two Horner chains each.)
 //  * sqrt_rsqrt(x) and rsqrt_pos(x): the hardware reciprocal square-root
 //    approximation refined by one third-order Newton step; the root as
 //    x * rsqrt with one residual correction.  x = 0 gives 0 (the reciprocal
@@ -72,26 +77,31 @@ __device__ __forceinline__ double exp_clamped(double x) {
 
 // Coefficients, read as constant-bank operands of the multiply-adds: as
 // literals each would cost two moves into registers per use.
-__constant__ double kExpSmall[13] = {0.5, 0.16666666666666613, 0.04166666666664616, 0.008333333333031724,
-                                     0.0013888888865815077, 0.0001984126878917537, 2.4801556448973442e-05,
-                                     2.755671130771333e-06, 2.7549086858331984e-07, 2.4975059697137715e-08,
-                                     2.0384099238823596e-09, 1.39778776896738e-10, 6.046017537551262e-12};
+__constant__ double kExpSmall[13] = {1.4426950408889634, 6755399441055744.0, 0.6931471805599453, 0.5000000000000001,
+                                     0.16666666666666669, 0.041666666666623824, 0.008333333333330039,
+                                     0.0013888888917367081, 0.00019841269863171557, 2.4801521057868204e-05,
+                                     2.7557268276905696e-06, 2.7620201591031547e-07, 2.5100472505694996e-08};
 __constant__ double kTanh01[16] = {1.0, -0.3333333333333273, 0.13333333333282113, -0.05396825395091773,
                                    0.021869488226930838, -0.008863232181130274, 0.003592104115230281,
                                    -0.00145571559077928, 0.0005896028950856166, -0.00023801236323479905,
                                    9.472256075732066e-05, -3.603918536997382e-05, 1.2306805295349983e-05,
                                    -3.402993826979274e-06, 6.496857637862531e-07, -6.20675330545365e-08};
 
-// e^x for x in [-1.5, 0]: 1 + x + x^2 q(x), q the degree-12 Chebyshev
-// interpolant of (e^x - 1 - x) / x^2 on the interval (error 1e-16)
+// e^x for x in [-1.5, 0]: x = k ln 2 + r, k = 0, -1, -2, and 2^k (1 + r +
+// r^2 q(r)), q the degree-9 interpolant of (e^r - 1 - r) / r^2 (error 1e-16 of
+// q, 2e-17 of the sum).  Relative error below 2^-52 (0.71 of it measured).  As
+// many FP64 operations as one polynomial 1 + x + x^2 q(x) over the whole
+// interval, whose terms cancel near -1.5 (6.1 of 2^-52 there).
 __device__ __forceinline__ double exp_small(double x) {
-    const double x2 = x * x;
-    double a = kExpSmall[12], b = kExpSmall[11];
+    const double t = fma(x, kExpSmall[0], kExpSmall[1]);
+    const double r = fma(t - kExpSmall[1], -kExpSmall[2], x), r2 = r * r;
+    double a = kExpSmall[11], b = kExpSmall[12];
 #pragma unroll
-    for (int k = 10; k >= 0; k -= 2) a = fma(a, x2, kExpSmall[k]);
+    for (int n = 9; n >= 3; n -= 2) a = fma(a, r2, kExpSmall[n]);
 #pragma unroll
-    for (int k = 9; k >= 1; k -= 2) b = fma(b, x2, kExpSmall[k]);
-    return 1.0 + fma(fma(b, x, a), x2, x);
+    for (int n = 10; n >= 4; n -= 2) b = fma(b, r2, kExpSmall[n]);
+    const double p = 1.0 + fma(fma(b, r, a), r2, r);
+    return __hiloint2double(__double2hiint(p) + (int)((unsigned)__double2loint(t) << 20), __double2loint(p));
 }
 
 // tanh(u) for u in [0, 1]: u p(u^2), p the degree-15 Chebyshev interpolant of

@@ -378,8 +378,9 @@ def dEdLat_to_stress(lat, dEdLat):
 
 
 def debug_math(which: int, x) -> np.ndarray:
-    """The branch-free FP64 exp (0), tanh on [0, 1] (1), sqrt (2) and 1/sqrt
-    (3) of the symmetry-function kernels, evaluated on the current device."""
+    """The branch-free FP64 exp (0), tanh on [0, 1] (1), sqrt (2), 1/sqrt (3)
+    and exp on [-1.5, 0] (4) and [-700, 0] (5) of the symmetry-function
+    kernels, evaluated on the current device."""
     x = np.ascontiguousarray(x, dtype=np.float64)
     y = np.empty_like(x)
     _check(lib().hdnnp_debug_math(which, x.size, _dp(x), _dp(y)))

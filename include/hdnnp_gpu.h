@@ -269,9 +269,9 @@ int hdnnp_last_launch_count(hdnnp_ctx* c, int* launches);
 /* The branch-free FP64 functions that the symmetry-function kernels use for
  * their bounded arguments, evaluated on the current device: y[i] = f(x[i]),
  * which = 0 exp (arguments clamped to [-708, 709]), 1 tanh (u in [0, 1]),
- * 2 sqrt, 3 1/sqrt.  No reference counterpart (a test hook; the reference
- * calls the Fortran intrinsics exp, tanh and sqrt in
- * symmetryFunctions.f90:201-327).                                            */
+ * 2 sqrt, 3 1/sqrt, 4 exp (x in [-1.5, 0]), 5 exp (x in [-700, 0]).  No
+ * reference counterpart (a test hook; the reference calls the Fortran
+ * intrinsics exp, tanh and sqrt in symmetryFunctions.f90:201-327).           */
 int hdnnp_debug_math(int which, int n, const double* x, double* y);
 
 /* ---------------------------------------------------------------- profiling

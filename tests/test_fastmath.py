@@ -1,13 +1,13 @@
 """The branch-free FP64 exp, tanh and square roots of csrc/fastmath.cuh.
 
-CPU: the exponential's operations (Cody-Waite reduction against ln 2, the
-degree-13 Taylor polynomial in Estrin form, the exponent-field scale) are
-emulated with exact fused multiply-adds, with the constants read from the
-header, and held against libm: within 1 ulp.  GPU: the device functions
-(hdnnp_debug_math) against numpy's libm results: exp and 1/sqrt within 2 ulp,
-sqrt within 1 ulp, tanh on [0, 1] within 6e-16 absolute (the subtraction
-1 - e^(-2u) keeps the absolute, not the relative error of e^(-2u); the
-cutoff function tanh^3 and its derivative vanish as u -> 0).  These replace the
+CPU: the exponentials' operations (Cody-Waite reduction against ln 2; the
+degree-13 Taylor polynomial in Estrin form, or the degree-9 interpolant of the
+form for [-1.5, 0]; the exponent-field scale) are emulated with exact fused
+multiply-adds, with the constants read from the header, and held against libm
+or its 80-bit form: within 1 ulp, 2^-52 relative on [-1.5, 0].  GPU: the
+device functions (hdnnp_debug_math) against numpy's results: exp and 1/sqrt
+within 2 ulp, sqrt within 1 ulp, exp on [-1.5, 0] within 2^-52 and tanh on
+[0, 1] (u times a polynomial in u^2) within 4e-16 relative.  These replace the
 library calls of the reference's intrinsics exp, tanh and sqrt
 (symmetryFunctions.f90:201-327) in the symmetry-function kernels.
 """
@@ -99,3 +99,71 @@ def test_device_functions_against_libm(pkg):
     # bad selector
     with pytest.raises(engine.HdnnpError):
         engine.debug_math(7, x[:4])
+
+
+def _table(name):
+    src = open(HEADER).read()
+    body = src[src.index(f"__constant__ double {name}["):]
+    return [float(v) for v in re.findall(r"-?[0-9.]+(?:e[+-]?[0-9]+)?", body[body.index("{"): body.index("}")])]
+
+
+def _exp_small_emulated(x, c):
+    t = _fma(x, c[0], c[1])
+    kd = t - c[1]
+    r = _fma(kd, -c[2], x)
+    r2 = r * r
+    a, b = c[11], c[12]
+    for n in (9, 7, 5, 3):
+        a = _fma(a, r2, c[n])
+    for n in (10, 8, 6, 4):
+        b = _fma(b, r2, c[n])
+    return math.ldexp(1.0 + _fma(_fma(b, r, a), r2, r), int(kd))
+
+
+def _bounded_arguments(lo, n, seed):
+    """[lo, 0] with both ends and the borders of the reduction."""
+    rng = np.random.default_rng(seed)
+    k = np.arange(0.5, -lo / math.log(2.0)) * math.log(2.0)
+    x = np.concatenate([lo * rng.random(n), -rng.random(n // 10) * 1e-3, [lo, 0.0, -1e-300], -k, -k * (1 + 1e-15),
+                        -k * (1 - 1e-15)])
+    return x[x >= lo]
+
+
+def test_exp_small_emulation():
+    """Reduction (error of ln 2 in one double, rounding of r), the last terms
+    of the polynomial and the last addition: below 2^-52 relative."""
+    c = _table("kExpSmall")
+    assert len(c) == 13
+    for x in _bounded_arguments(-1.5, 3000, 3):
+        ref = Fraction(*np.exp(np.longdouble(x)).as_integer_ratio())
+        assert abs(Fraction(_exp_small_emulated(float(x), c)) - ref) <= ref / 2**52, x
+
+
+def test_exp_neg_coefficients():
+    """exp_neg's table holds exp_clamped's constants and 1/n!, n = 2..13."""
+    K, Q = _exp_constants()
+    c = _table("kExpNeg")
+    assert c[:4] == [K["kLog2e"], K["kShift"], K["kLn2Hi"], K["kLn2Lo"]]
+    assert c[4:] == [v for a, b in Q for v in (b, a)]
+
+
+@pytest.mark.gpu
+def test_device_bounded_functions(pkg):
+    """The forms without range tests: exp on [-1.5, 0] below 2^-52 relative,
+    exp on [-700, 0] within 2 ulp; tanh on [0, 1] within 4e-16 relative (the
+    two last roundings of the polynomial, the product and the interpolation,
+    also as u -> 0)."""
+    from hdnnp_b200 import engine
+
+    def err(y, ref):
+        return np.abs((y.astype(np.longdouble) - ref) / ref).astype(float).max()
+
+    x = _bounded_arguments(-1.5, 100000, 4)
+    assert err(engine.debug_math(4, x), np.exp(x.astype(np.longdouble))) <= 2.0**-52
+    x = _bounded_arguments(-700.0, 100000, 5)
+    y = engine.debug_math(5, x)
+    assert (np.abs(y - np.exp(x)) / np.spacing(np.exp(x))).max() <= 2.0
+    rng = np.random.default_rng(6)
+    u = np.concatenate([rng.random(100000), 10.0 ** -rng.uniform(0, 12, 2000), [1.0, 1e-300]])
+    assert err(engine.debug_math(1, u), np.tanh(u.astype(np.longdouble))) <= 4e-16
+    assert engine.debug_math(1, np.zeros(1))[0] == 0.0
