@@ -580,9 +580,8 @@ int upload_model(hdnnp_model* m) {
     std::vector<double2> pscale(pmap.size(), double2{0.0, 0.0});
     for (size_t q = 0; D.fast && q < pmap.size(); ++q) {
         if (pmap[q] < 0) continue;
-        const int P = fast_shape_p(D.fast), NZ = kFastShapes[D.fast][1], NE = kFastShapes[D.fast][2];
-        const size_t at = q / ((size_t)nblk * P) * nsf_max + pmap[q];
-        pscale[q] = double2{D.pfz[(q % P) / NE % NZ] * sinvw[at], -smean[at] * sinvw[at]};
+        const size_t at = q / ((size_t)nblk * fast_shape_p(D.fast)) * nsf_max + pmap[q];
+        pscale[q] = double2{-smean[at], sinvw[at]};
     }
     size_t o_ps = add(pscale.data(), pscale.size() * sizeof(double2));
     size_t o_pm = add(pmap.data(), pmap.size() * sizeof(short)), o_wf = add(wf.data(), wf.size() * 4),

@@ -100,7 +100,7 @@ struct DevModel {
     int g4_full;              // 1 when every centre element has angular functions for every element pair
     int zmaxbit;              // highest bit of the integer zeta - 1 values
     const short* pmap;        // [nel][nblk][P]: SF index of product entry p, or -1
-    const double2* pscale;    // [nel][nblk][P]: G = x * sum + y (2^(1-zeta) / width, -mean / width)
+    const double2* pscale;    // [nel][nblk][P]: G = (pfz * sum + x) * y (x = -mean, y = 1 / width)
     // FP32 copies of the network weights (mixed-precision form)
     const float* wf;
     const float* wtf;

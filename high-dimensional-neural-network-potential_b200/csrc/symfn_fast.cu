@@ -1004,7 +1004,8 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocksV<T>) k_sfv_fast(Batch b, 
                                             const size_t at = ((size_t)c * nblk + t) * P + row * NE + col % NE;
                                             const int sf = m.pmap[at];
                                             const double2 q = m.pscale[at];
-                                            if (sf >= 0) Gi[sf] = (T)fma(q.x, acc[g][mt][v], q.y);
+                                            // the difference to the mean before the division by the width
+                                            if (sf >= 0) Gi[sf] = (T)(fma(m.pfz[row % NZ], acc[g][mt][v], q.x) * q.y);
                                         }
                                         acc[g][mt][v] = 0.0;
                                     }

@@ -121,3 +121,37 @@ def test_forms_need_no_list(pkg, W, tmp_path):
             assert r[0] == res[0][0] and np.array_equal(r[1], res[0][1]) and np.array_equal(r[2], res[0][2])
     finally:
         pot.close()
+
+
+def test_value_at_its_mean_scales_to_zero(pkg, tmp_path):
+    """(value - mean) / (max - min) with the mean set to the value: the
+    difference is formed first, so the scaled function is exactly zero."""
+    from hdnnp_b200 import engine
+
+    Z = np.array([1, 6, 7, 53, 82], np.int32)  # an atom of every element
+    pos = np.array([[0.0, 0, 0], [3, 1, 0.2], [1, 3, 2.5], [-2, 2, 4], [2.5, -2, -3]])
+    scaling = tmp_path / "scaling.data"
+    write_potential(tmp_path, (0.001, 0.01), (1, 2, 4, 16))
+
+    def values():
+        pot = engine.Hdnnp.from_runner(str(tmp_path))
+        try:
+            pot.set_option("small_eval", 0)
+            pot.energy_and_forces(engine.AtStruct(Z, pos, None))
+            nsf = max(pot.nsf.values())
+            return pot.fetch("G", len(Z) * nsf).reshape(len(Z), nsf), [pot.nsf[int(z)] for z in Z]
+        finally:
+            pot.close()
+
+    n = [sum(1 for x in scaling.read_text().splitlines() if x.split()[0] == str(k + 1) and len(x.split()) == 5)
+         for k in range(5)]
+    rows = [(e + 1, k + 1) for e in range(5) for k in range(n[e])]
+    scaling.write_text("\n".join(f"{e} {k} 0.0 1.0 0.0" for e, k in rows) + "\n-1.0 1.0\n")
+    raw, nsf = values()
+    assert nsf == n and np.count_nonzero(raw[:, : min(n)]) > 500
+    w = np.random.default_rng(2).uniform(0.1, 3.0, len(rows))
+    scaling.write_text("\n".join(f"{e} {k} 0.0 {x:.17g} {raw[e - 1, k - 1]:.17g}" for (e, k), x in zip(rows, w))
+                       + "\n-1.0 1.0\n")
+    scaled, _ = values()
+    for a in range(5):
+        assert np.count_nonzero(scaled[a, : n[a]]) == 0
