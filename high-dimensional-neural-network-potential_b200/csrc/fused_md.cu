@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_md(DevModel m, TinyArg
                 continue;
             }
             const size_t k = (size_t)c * nsf + sf;
-            G[(size_t)i * nsf + sf] = (acc - m.smean[k]) * m.sinvw[k];
+            G[(size_t)i * nsf + sf] = (acc - m.smean[k]) / m.swidth[k];
         }
         __syncthreads();
         // networks: one (atom, neuron) per thread and layer; activations in mlp
@@ -761,7 +761,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_md(DevModel m, TinyArg
                     double s = 0.0;
                     for (int o = 0; o < wout; ++o) s += da[o] * Wm[(size_t)o * wi + k];
                     if (l == 0)
-                        Wt[(size_t)i * nsf + k] = s * m.sinvw[(size_t)e * nsf + k];
+                        Wt[(size_t)i * nsf + k] = s / m.swidth[(size_t)e * nsf + k];
                     else
                         d1[x] = s * act_d(m.act[l - 1], cp[x], yp[x]);
                 }

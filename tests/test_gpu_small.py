@@ -155,3 +155,33 @@ def test_resident_kernel_serves_calls(eng, c1):
         pot.close()  # the resident kernel is waiting: freeing the context stops it
         assert time.perf_counter() - t0 < 1.0
         ref.close()
+
+
+def write_hydrogen(d, functions, scaling):
+    """One element, the given symmetry functions, a linear network: the energy
+    is the sum of the scaled functions."""
+    (d / "input.nn").write_text("\n".join([
+        "number_of_elements 1", "elements H", "global_hidden_layers_short 0", "global_activation_short l",
+        "cutoff_type 2", "scale_symmetry_functions", "center_symmetry_functions"]
+        + [f"symfunction_short H {f}" for f in functions]) + "\n")
+    (d / "scaling.data").write_text("".join(f"1 {k + 1} 0.0 {w!r} {mean!r}\n" for k, (w, mean) in enumerate(scaling))
+                                    + "-1.0 1.0\n")
+    (d / "weights.001.data").write_text("1.0\n" * len(functions) + "0.0\n")
+
+
+def test_scaling_divides_by_the_width(eng, tmp_path):
+    """H2 with one radial function: the energy is twice the correctly rounded
+    quotient of the value by the width."""
+    pos = np.array([[0.0, 0, 0], [1.1, 0.7, -0.4]])
+
+    def value(width):
+        write_hydrogen(tmp_path, ["2 H 0.05 0.3 12.0"], [(width, 0.0)])
+        pot = eng.Hdnnp.from_runner(str(tmp_path))
+        try:
+            return 0.5 * pot.energy_and_forces(eng.AtStruct(np.array([1, 1], np.int32), pos))[0]
+        finally:
+            pot.close()
+
+    v = value(1.0)
+    for w in np.random.default_rng(1).uniform(0.1, 3.0, 40).tolist():
+        assert value(w) == v / w
