@@ -648,7 +648,9 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_md(DevModel m, TinyArg
             sqrt_rsqrt(rjk2, rjk, irjk);
             tiny_cutoff(rjk, irjk, 1.0 / mrc, mrc, fjk, dfjk);
             const double t1 = -1.0 / (rj * rk);
-            const double cth = 0.5 * (rjk * rjk - rj * rj - rk * rk) * t1;
+            // by the product of the vectors: the three squares of the
+            // distances cancel (r_ij << r_ik)
+            const double cth = -(aj[0] * ak[0] + aj[1] * ak[1] + aj[2] * ak[2]) * t1;
             const double fcp = aj[4] * ak[4] * fjk;
             double* s = ps + 5 * (size_t)P;
             s[0] = fjk;

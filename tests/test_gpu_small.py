@@ -185,3 +185,25 @@ def test_scaling_divides_by_the_width(eng, tmp_path):
     v = value(1.0)
     for w in np.random.default_rng(1).uniform(0.1, 3.0, 40).tolist():
         assert value(w) == v / w
+
+
+def test_right_angle_has_no_cosine(eng, tmp_path):
+    """A right angle with legs of very different length: the functions with
+    lambda = 1 and -1 agree to the last bit (their difference is the energy;
+    the outer atoms' functions have no weight)."""
+    (tmp_path / "input.nn").write_text("\n".join([
+        "number_of_elements 2", "elements H O", "global_hidden_layers_short 0", "global_activation_short l",
+        "cutoff_type 2", "symfunction_short H 3 O O 0.001 1.0 1.0 12.0", "symfunction_short H 3 O O 0.001 -1.0 1.0 12.0",
+        "symfunction_short O 2 H 0.05 0.0 12.0"]) + "\n")
+    (tmp_path / "scaling.data").write_text("1 1 0.0 1.0 0.0\n1 2 0.0 1.0 0.0\n2 1 0.0 1.0 0.0\n-1.0 1.0\n")
+    (tmp_path / "weights.001.data").write_text("1.0\n-1.0\n0.0\n")
+    (tmp_path / "weights.008.data").write_text("0.0\n0.0\n")
+    pot = eng.Hdnnp.from_runner(str(tmp_path))
+    try:
+        rng = np.random.default_rng(3)
+        for a, b in zip(rng.uniform(0.5, 2.0, 50), rng.uniform(6.0, 10.0, 50)):
+            pos = np.array([[0.0, 0, 0], [a, 0, 0], [0, b, 0]])
+            E, F, _ = pot.energy_and_forces(eng.AtStruct(np.array([1, 8, 8], np.int32), pos))
+            assert E == 0.0 and np.abs(F).max() > 0.0
+    finally:
+        pot.close()
