@@ -416,7 +416,7 @@ __device__ __forceinline__ int owner_of(const int* off, int n, int x) {
 __device__ __forceinline__ void tiny_cutoff(double r, double ir, double irc, double rc, double& fc, double& dfc) {
     fc = dfc = 0.0;
     if (r < rc) {
-        const double t = tanh01(1.0 - r * irc), tt = t * t;
+        const double t = tanh01((rc - r) * irc), tt = t * t;  // (rc - r exact near rc, where r / rc rounds most)
         fc = tt * t;
         dfc = -3.0 * irc * ir * (tt - tt * tt);
     }

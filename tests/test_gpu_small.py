@@ -207,3 +207,18 @@ def test_right_angle_has_no_cosine(eng, tmp_path):
             assert E == 0.0 and np.abs(F).max() > 0.0
     finally:
         pot.close()
+
+
+def test_cutoff_near_its_end(eng, tmp_path):
+    """H2 at distances that are exact in binary, up to just inside the cutoff:
+    the energy is 2 tanh^3(1 - r / rc) to the rounding of a few operations
+    (3e-15 relative), not of the quotient r / rc (1e-16 / (1 - r / rc))."""
+    write_hydrogen(tmp_path, ["2 H 0.0 0.0 12.0"], [(1.0, 0.0)])
+    pot = eng.Hdnnp.from_runner(str(tmp_path))
+    try:
+        for r in 12.0 - np.concatenate([np.arange(1, 65) / 1024, np.arange(1, 40) / 4]):
+            E, _, _ = pot.energy_and_forces(eng.AtStruct(np.array([1, 1], np.int32), np.array([[0.0, 0, 0], [0, 0, r]])))
+            ref = 2 * np.tanh((12 - np.longdouble(r)) / 12) ** 3
+            assert abs(E - ref) <= 3e-15 * ref, r
+    finally:
+        pot.close()
