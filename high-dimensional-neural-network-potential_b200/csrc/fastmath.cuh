@@ -139,6 +139,12 @@ __device__ __forceinline__ double exp_neg(double x) {
     return p * __hiloint2double((k + 1023) << 20, 0);
 }
 
+// x^y, y not an integer, of an angular function's base x = 1 + lambda cos: a
+// base that rounding takes below zero (collinear atoms, lambda = 1 or -1) is
+// zero, not NaN.  The limits lie above the rounding of the cosine.
+__device__ __forceinline__ double base_pow(double x, double y) { return pow(x < 0.0 && x > -1e-10 ? 0.0 : x, y); }
+__device__ __forceinline__ float base_pow(float x, float y) { return powf(x < 0.0f && x > -1e-4f ? 0.0f : x, y); }
+
 // 1 / sqrt(x) for x > 0 (x = 0 gives 1e150)
 __device__ __forceinline__ double rsqrt_pos(double x) {
     // max(x, 1e-300) on the high word (x >= 0; the low word only matters above)

@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_md(DevModel m, TinyArg
             const double rsum = aj[3] * aj[3] + ak[3] * ak[3] + (cx * cx + cy * cy + cz * cz);
             const double base = 1.0 + f.lambda * ps[5 * (size_t)P + 3];
             pe[x] = exp_clamped(-f.eta * rsum);
-            pt[x] = f.izeta >= 0 ? ipow(base, f.izeta - 1) : pow(base, f.zeta - 1.0);
+            pt[x] = f.izeta >= 0 ? ipow(base, f.izeta - 1) : base_pow(base, f.zeta - 1.0);
         }
         __syncthreads();
         // symmetry-function values, one (atom, function) per thread

@@ -255,7 +255,6 @@ __device__ __forceinline__ float xexp(float x) { return __expf(x); }
 // tanh of a cutoff argument u = 1 - r/rc in [0, 1]
 __device__ __forceinline__ double xtanh(double x) { return tanh01(x); }
 __device__ __forceinline__ float xtanh(float x) { return tanhf(x); }
-__device__ __forceinline__ double xpow(double x, double y) { return pow(x, y); }
 
 // exp of an angular -eta r^2 and of a radial -eta (r - rs)^2.  kB: every
 // argument of the potential's functions is in the range of the functions
@@ -614,10 +613,10 @@ __device__ __forceinline__ void powers(const DevModel& m, T X, T (&Tz)[S::NZ], T
             if (z < m.fz) {
                 const int ez = m.zint[z];
                 if (kDeriv) {
-                    p = ez >= 0 ? rpow(ch, ez) : xpow(X, (T)m.zet[z] - (T)1);
+                    p = ez >= 0 ? rpow(ch, ez) : base_pow(X, (T)m.zet[z] - (T)1);
                     q = p * X;
                 } else {
-                    q = ez >= 0 ? rpow(ch, ez + 1) : xpow(X, (T)m.zet[z]);
+                    q = ez >= 0 ? rpow(ch, ez + 1) : base_pow(X, (T)m.zet[z]);
                 }
             }
             Tz[z] = q;
@@ -681,11 +680,11 @@ __device__ __forceinline__ void powers2(const DevModel& m, float2 X, float2 (&Tz
                     }
                 } else if (kDeriv) {
                     const float zm = (float)m.zet[z] - 1.0f;
-                    p = make_float2(powf(X.x, zm), powf(X.y, zm));
+                    p = make_float2(base_pow(X.x, zm), base_pow(X.y, zm));
                     q = __fmul2_rn(p, X);
                 } else {
                     const float zz = (float)m.zet[z];
-                    q = make_float2(powf(X.x, zz), powf(X.y, zz));
+                    q = make_float2(base_pow(X.x, zz), base_pow(X.y, zz));
                 }
             }
             Tz[z] = q;

@@ -7,6 +7,7 @@
 #pragma once
 
 #include "engine.h"
+#include "fastmath.cuh"
 
 namespace hdnnp {
 
@@ -332,7 +333,7 @@ __device__ __forceinline__ void sfv_atom(const Batch& b, const DevModel& m, int 
                                     last_eta = f.eta;
                                 }
                                 const double base = 1.0 + f.lambda * cth;
-                                const double t2 = f.izeta >= 0 ? ipow(base, f.izeta - 1) : pow(base, f.zeta - 1.0);
+                                const double t2 = f.izeta >= 0 ? ipow(base, f.izeta - 1) : base_pow(base, f.zeta - 1.0);
                                 acc[u] += f.pf * (t2 * base) * ex * fcp;
                             }
                         }
@@ -457,7 +458,7 @@ __device__ __forceinline__ void sfg_atom(const Batch& b, const DevModel& m, int 
                             last_eta = f.eta;
                         }
                         const double base = 1.0 + f.lambda * cth;
-                        const double t2 = f.izeta >= 0 ? ipow(base, f.izeta - 1) : pow(base, f.zeta - 1.0);
+                        const double t2 = f.izeta >= 0 ? ipow(base, f.izeta - 1) : base_pow(base, f.zeta - 1.0);
                         const double wpe = s.w[f.sf] * f.pf * ex;
                         const double cp = t2 * base;
                         A += wpe * cp;

@@ -155,3 +155,36 @@ def test_value_at_its_mean_scales_to_zero(pkg, tmp_path):
     scaled, _ = values()
     for a in range(5):
         assert np.count_nonzero(scaled[a, : n[a]]) == 0
+
+
+@pytest.mark.parametrize("small, generic, prec", [(1, 0, "FP64"), (0, 0, "FP64"), (0, 1, "FP64"), (0, 0, "MIXED")])
+def test_collinear_atoms_with_noninteger_zeta(pkg, tmp_path, small, generic, prec):
+    """1 + lambda cos of three atoms in a line is zero up to the sign of its
+    rounding: finite results, equal to those of a bend of 1e-4 Bohr (the
+    energy changes by about its square, the forces by its curvature)."""
+    from hdnnp_b200 import engine
+
+    write_potential(tmp_path, (0.001, 0.01), (1, 2.5, 6.3))
+    pot = engine.Hdnnp.from_runner(str(tmp_path))
+    try:
+        pot.set_option("small_eval", small)
+        pot.set_option("generic_sf", generic)
+        pot.set_precision(getattr(engine, "HDNNP_PREC_" + prec))
+        rng = np.random.default_rng(0)
+        zs = sorted(int(z) for z in pot.nsf)
+        for k in range(60):
+            v = np.array([1.0, 0, 0]) if k % 4 < 2 else rng.normal(size=3)
+            v /= np.linalg.norm(v)
+            w = np.cross(v, rng.normal(size=3))
+            w /= np.linalg.norm(w)
+            d1, d2 = rng.uniform(1.5, 4.0, 2)
+            pos = np.array([-d1 * v, 0 * v, (d1 if k % 2 else d2) * v])
+            Z = rng.choice(zs, 3).astype(np.int32)
+            E, F, _ = pot.energy_and_forces(engine.AtStruct(Z, pos))
+            assert np.isfinite(E) and np.isfinite(F).all(), k
+            pos[1] += 1e-4 * w
+            E1, F1, _ = pot.energy_and_forces(engine.AtStruct(Z, pos))
+            assert abs(E - E1) <= (1e-6 if prec == "FP64" else 1e-4), k
+            assert np.abs(F - F1).max() <= 1e-3 * max(1.0, np.abs(F).max()), k
+    finally:
+        pot.close()
