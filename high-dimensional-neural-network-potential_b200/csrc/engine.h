@@ -19,6 +19,17 @@ namespace hdnnp {
 
 constexpr int kMaxEl = 16;
 
+// Dynamic shared memory of a block (227 KB), and the limit that every kernel
+// with more than 48 KB of it is given: always the same one, whatever the
+// launch needs.  A kernel has one limit per device, so one launch's smaller
+// value would refuse another's launch, of a larger model or molecule, from
+// this thread or another.  fixed: bytes of static shared memory.
+constexpr int kSmemLimit = 227 * 1024;
+template <typename K>
+inline void raise_smem_limit(K kernel, size_t smem, int fixed = 0) {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit - fixed);
+}
+
 // Per-structure set-up computed on the host in FP64 (same formulas as the
 // reference: artificial box for molecules, grid of >= 0.6 rc cells, search
 // range getNcells(grid, rc)).

@@ -22,7 +22,6 @@
 // Neighbours are listed in atom-index order (the reference walks its cell
 // grid; for a molecule both give the same set, the sums differ only in
 // rounding).
-#include <atomic>
 
 #include "engine.h"
 #include "fastmath.cuh"
@@ -961,7 +960,7 @@ int launch_small_resident(const DevModel& m, int natoms, ResidentBox* box, cudaS
     ta.elem = box->elem;
     ta.eval_only = 1;
     ta.box = box;
-    cudaFuncSetAttribute(k_tiny_md, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
+    raise_smem_limit(k_tiny_md, tsm);
     k_tiny_md<<<1, kTinyThreads, tsm, s>>>(m, ta);
     return 1;
 }
@@ -988,22 +987,7 @@ int launch_small_md(const Batch& b, const DevModel& m, const SmallMdArgs& x, cud
             for (int q = 0; q < 3 * x.natoms; ++q) ta.in_pos[q] = x.inline_pos[q];
             for (int i = 0; i < x.natoms; ++i) ta.in_elem[i] = x.inline_elem[i];
         }
-        // the shared-memory limit is raised once per device and size (the
-        // attribute call costs about a microsecond)
-        {
-            constexpr int kMaxDev = 64;
-            static std::atomic<size_t> raised[kMaxDev];
-            int dev = 0;
-            cudaGetDevice(&dev);
-            if (dev < 0 || dev >= kMaxDev || raised[dev].load(std::memory_order_relaxed) < tsm) {
-                cudaFuncSetAttribute(k_tiny_md, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
-                if (dev >= 0 && dev < kMaxDev) {
-                    size_t cur = raised[dev].load(std::memory_order_relaxed);
-                    while (cur < tsm && !raised[dev].compare_exchange_weak(cur, tsm)) {
-                    }
-                }
-            }
-        }
+        raise_smem_limit(k_tiny_md, tsm);
         k_tiny_md<<<1, kTinyThreads, tsm, s>>>(m, ta);
         return 1;
     }
@@ -1022,7 +1006,7 @@ int launch_small_md(const Batch& b, const DevModel& m, const SmallMdArgs& x, cud
     a.acc = x.acc;
     a.eval_only = x.eval_only;
     auto run = [&](auto kernel) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        raise_smem_limit(kernel, smem, sizeof(unsigned long long) * kSmallMolecule);
         kernel<<<1, kThreads, smem, s>>>(b, m, a);
     };
     if (m.gmax <= 4)

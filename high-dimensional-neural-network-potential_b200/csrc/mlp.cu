@@ -610,7 +610,7 @@ void run_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     for (int l = 0; l < m.nlayers; ++l)
         if (m.width[l + 1] > maxw) maxw = m.width[l + 1];
     size_t smem = mlp_smem_bytes(m, sizeof(T));
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_mlp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    raise_smem_limit(k_mlp<T>, smem);
     int tiles = b.natoms / kTile + m.nel + 1;
     k_mlp<T><<<tiles, kThreads, smem, s>>>(b, m, maxw);
 }
@@ -623,9 +623,6 @@ void run_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
 // form).  Measured for 280-25-25-1 networks, split / resident: 93 / 88 us at
 // 18,000 atoms, 156 / 145 at 36,000.  Both give an atom the same bits.
 constexpr int kResidentTilesPerSm = 16;
-// dynamic shared memory of a block; always set as the kernels' limit (contexts
-// on other threads may launch them with other sizes)
-constexpr int kSmemLimit = 227 * 1024;
 
 int launch_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     if (!m.dm_ok) {
@@ -638,12 +635,12 @@ int launch_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     const int nsm = device_sm_count();
     if (rsm <= (size_t)kSmemLimit && b.natoms >= nsm * kResidentTilesPerSm * kDR) {
         auto k = (m.nsf_max & 1) ? k_mlp_resident<false> : k_mlp_resident<true>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+        raise_smem_limit(k, rsm);
         k<<<nsm, 32 * kRW, rsm, s>>>(b, m, nin);
         return 1;
     }
     const size_t smem = (size_t)split_doubles(m) * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_mlp_split, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    raise_smem_limit(k_mlp_split, smem);
     k_mlp_split<<<b.natoms / kDR + m.nel + 1, 32 * kDW, smem, s>>>(b, m);
     return 1;
 }

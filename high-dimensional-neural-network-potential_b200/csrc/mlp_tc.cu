@@ -518,7 +518,7 @@ size_t mlp_tc_smem_bytes(const DevModel& m) { return tc_plan(m).total; }
 template <int NL>
 void run_tc(const Batch& b, const DevModel& m, cudaStream_t s) {
     const size_t smem = tc_plan(m).total;
-    cudaFuncSetAttribute(k_mlp_tc<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    raise_smem_limit(k_mlp_tc<NL>, smem);
     const int tiles = b.natoms / kM + m.nel + 1;
     k_mlp_tc<NL><<<tiles, kThr, smem, s>>>(b, m);
 }

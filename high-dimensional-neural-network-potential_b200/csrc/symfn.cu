@@ -64,8 +64,7 @@ int num_sms() { return device_sm_count(); }
 template <int GM>
 void launch_values_gm(const Batch& b, const DevModel& m, int mm, cudaStream_t st) {
     size_t smem = warp_bytes<double>(mm, m.nsf_max, false) * kWarpsPerBlock;
-    // set on every launch: the attribute is per device, and calls come from several threads
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_sf_values<GM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    raise_smem_limit(k_sf_values<GM>, smem);
     int blocks = (b.natoms + kWarpsPerBlock - 1) / kWarpsPerBlock;
     int cap = num_sms() * 16;
     if (blocks > cap) blocks = cap;
@@ -93,7 +92,7 @@ int launch_sf_values(const Batch& b, const DevModel& m, cudaStream_t st) {
 int launch_sf_gradients(const Batch& b, const DevModel& m, cudaStream_t st) {
     const int mm = ((b.mmax + 31) / 32) * 32 > 0 ? ((b.mmax + 31) / 32) * 32 : 32;
     size_t smem = warp_bytes<double>(mm, m.nsf_max, true) * kWarpsPerBlock;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_sf_gradients, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    raise_smem_limit(k_sf_gradients, smem);
     int blocks = (b.natoms + kWarpsPerBlock - 1) / kWarpsPerBlock;
     int cap = num_sms() * 16;
     if (blocks > cap) blocks = cap;

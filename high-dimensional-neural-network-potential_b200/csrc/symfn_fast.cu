@@ -1387,15 +1387,6 @@ __global__ void k_list_wide(Batch b, int mm) {
 
 int nsm() { return device_sm_count(); }
 
-constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory of a block
-
-template <typename K>
-void set_smem(K kernel, size_t smem) {
-    // always the same value: contexts on other threads launch the same kernel
-    // with other sizes, and one's smaller limit must not meet another's launch
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
-}
-
 // Shared memory per warp grows with the largest neighbour count of the
 // batch, and it sets how many warps an SM holds.  Atoms with at most `split`
 // neighbours run in a launch sized for that count; the others are listed and
@@ -1422,24 +1413,24 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
     if (b.sf_split == 0 && mfull > split) {
         // a batch whose warps all fit on the GPU at the full size needs no
         // second launch (same code per atom: same results)
-        const int fit = std::min<int>(resident, (int)(kSmemMax / (warp_bytes(mfull) * kWarps)));
+        const int fit = std::min<int>(resident, (int)(kSmemLimit / (warp_bytes(mfull) * kWarps)));
         if ((long long)b.natoms <= (long long)nsm() * fit * kWarps) split = mfull;
     }
     int L = 0;
     auto go = [&](int mm, int part, cudaStream_t on) {
         // four warps a block, fewer where so many neighbours do not fit
         int nw = kWarps;
-        while (nw > 1 && warp_bytes(mm) * nw > kSmemMax) nw >>= 1;
+        while (nw > 1 && warp_bytes(mm) * nw > kSmemLimit) nw >>= 1;
         const size_t smem = warp_bytes(mm) * nw;
         int blocks = (b.natoms + nw - 1) / nw;
         const int cap = nsm() * (part == kPartWide ? kWideBlocksPerSm : per_sm);
         if (blocks > cap) blocks = cap;
         if (blocks < 1) blocks = 1;
         if (grad) {
-            set_smem(k_sfg_fast<T, S, kB>, smem);
+            raise_smem_limit(k_sfg_fast<T, S, kB>, smem);
             k_sfg_fast<T, S, kB><<<blocks, 32 * nw, smem, on>>>(b, m, mm, part);
         } else {
-            set_smem(k_sfv_fast<T, S, kB>, smem);
+            raise_smem_limit(k_sfv_fast<T, S, kB>, smem);
             k_sfv_fast<T, S, kB><<<blocks, 32 * nw, smem, on>>>(b, m, mm, part);
         }
         ++L;

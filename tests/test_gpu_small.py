@@ -222,3 +222,24 @@ def test_cutoff_near_its_end(eng, tmp_path):
             assert abs(E - ref) <= 3e-15 * ref, r
     finally:
         pot.close()
+
+
+def test_large_small_large_launches(eng):
+    """A large molecule by a launch, a smaller one through the resident
+    kernel, the large one again: one kernel, whose shared-memory limit stays
+    the largest."""
+    pot = eng.Hdnnp.from_runner(EXAMPLE_DIR)
+    try:
+        zs = sorted(int(z) for z in pot.nsf)
+        rng = np.random.default_rng(0)
+        pos = np.array([[3.0 * (i % 3), 3.0 * (i // 3 % 3), 3.0 * (i // 9)] for i in range(14)]) + rng.normal(0, 0.1, (14, 3))
+        Z = np.resize(np.array(zs, np.int32), 14)
+        first = {}
+        for n in (14, 3, 14, 8, 14):
+            for resident in (0, 1, 0):
+                pot.set_option("small_resident", resident)
+                E, F, _ = pot.energy_and_forces(eng.AtStruct(Z[:n], pos[:n]))
+                e, f = first.setdefault(n, (E, F))
+                assert E == e and np.array_equal(F, f)
+    finally:
+        pot.close()
