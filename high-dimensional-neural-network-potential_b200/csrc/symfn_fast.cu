@@ -1394,10 +1394,14 @@ int nsm() { return device_sm_count(); }
 // context's side stream (after it, the few listed atoms took 80 of the 440 us
 // of each pass for 96 structures, one atom's latency on a nearly idle GPU).
 // Each atom is evaluated once, by the same code.
+// Both launches have the same grid: in a dense batch nearly every atom is
+// listed (19,200 atoms with 95-111 neighbours, 5 elements, values / gradients
+// in ms: 1.57 / 2.90 FP64 and 1.21 / 1.58 mixed; with two blocks per SM of
+// the listed atoms 2.23 / 4.59 and 1.87 / 2.48).
 // The split and the persistent grid (blocks per SM) are the knobs of the
 // plans' autotuner (Batch::sf_split, Batch::sf_blocks_per_sm).
 constexpr int kBlocksPerSm = 32;
-constexpr int kWideBlocksPerSm = 2;  // of the launch for the listed atoms
+constexpr size_t kSmemSm = 228 * 1024;  // shared memory of an SM; 1 KB of every block is the system's
 
 template <typename T, class S, bool kB>
 int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
@@ -1406,24 +1410,45 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
     // default split: the largest count at which the blocks the registers
     // allow still fit (1 KB of every block is the system's)
     const int resident = grad ? kBlocksG<T> : kBlocksV<T>;
+    // Warps per block at neighbour count mm and the warps that an SM then
+    // holds: four, or fewer where a block of four leaves more than an eighth
+    // of that number unused (160 neighbours, FP64 gradients: 4 warps an SM in
+    // one block, 7 in blocks of one; the dense batch above 4.62 -> 2.90 ms).
+    // For one warp more the smaller blocks do not pay: they take the places
+    // of the other launch's blocks (758,676 atoms, 12 -> 13 and 8 -> 9 warps:
+    // 31.8 -> 32.5 ms per step).
+    auto warps_per_block = [&](int mm, int& on_sm) {
+        int best = 1;
+        on_sm = 0;
+        for (int nw = kWarps; nw >= 1; nw >>= 1) {
+            const size_t block = warp_bytes(mm) * nw;
+            if (block > (size_t)kSmemLimit) continue;
+            const int n = nw * (int)std::min<size_t>(resident * kWarps / nw, kSmemSm / (block + 1024));
+            if (8 * n > 9 * on_sm) {
+                best = nw;
+                on_sm = n;
+            }
+        }
+        return best;
+    };
     int fitting = 32;
-    while (fitting + 8 <= 1024 && (warp_bytes(fitting + 8) * kWarps + 1024) * resident <= 228 * 1024) fitting += 8;
+    while (fitting + 8 <= 1024 && (warp_bytes(fitting + 8) * kWarps + 1024) * resident <= kSmemSm) fitting += 8;
     int split = b.sf_split > 0 ? (b.sf_split + 7) / 8 * 8 : b.sf_split < 0 ? mfull : fitting;
     const int per_sm = b.sf_blocks_per_sm > 0 ? b.sf_blocks_per_sm : kBlocksPerSm;
     if (b.sf_split == 0 && mfull > split) {
         // a batch whose warps all fit on the GPU at the full size needs no
         // second launch (same code per atom: same results)
-        const int fit = std::min<int>(resident, (int)(kSmemLimit / (warp_bytes(mfull) * kWarps)));
-        if ((long long)b.natoms <= (long long)nsm() * fit * kWarps) split = mfull;
+        int fit;
+        warps_per_block(mfull, fit);
+        if ((long long)b.natoms <= (long long)nsm() * fit) split = mfull;
     }
     int L = 0;
     auto go = [&](int mm, int part, cudaStream_t on) {
-        // four warps a block, fewer where so many neighbours do not fit
-        int nw = kWarps;
-        while (nw > 1 && warp_bytes(mm) * nw > kSmemLimit) nw >>= 1;
+        int fit;
+        const int nw = warps_per_block(mm, fit);
         const size_t smem = warp_bytes(mm) * nw;
         int blocks = (b.natoms + nw - 1) / nw;
-        const int cap = nsm() * (part == kPartWide ? kWideBlocksPerSm : per_sm);
+        const int cap = nsm() * per_sm * kWarps / nw;
         if (blocks > cap) blocks = cap;
         if (blocks < 1) blocks = 1;
         if (grad) {
