@@ -833,16 +833,20 @@ int run_pipeline(hdnnp_ctx* c, int nstruct, int natoms, const int32_t* Zd, const
     fast = D.fast && !c->generic_sf;
     mixed = c->precision == HDNNP_PREC_MIXED && fast;
     if (fast) {
-        if ((r = c->pairs.ensure(N * (size_t)kPairCap)) || (r = c->npairs.ensure(N)) ||
-            (r = c->wide.ensure(N + 1)))
-            return r;
-        if (!c->side) CUDA_TRY(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-        for (auto* e : {&c->fork, &c->join})
-            if (!*e) CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-        b.wide = c->wide.p;
-        b.side = c->side;
-        b.fork = c->fork;
-        b.join = c->join;
+        if ((r = c->pairs.ensure(N * (size_t)kPairCap)) || (r = c->npairs.ensure(N))) return r;
+        // the list of the atoms of the second launch and the stream beside
+        // (60-700 us to create) when a batch first has such atoms; a plan's
+        // probe evaluation has the launch shapes of its captured ones
+        if (sf_fast_lists_atoms(b, D, mixed)) {
+            if ((r = c->wide.ensure(N + 1))) return r;
+            if (!c->side) CUDA_TRY(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+            for (auto* e : {&c->fork, &c->join})
+                if (!*e) CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+            b.wide = c->wide.p;
+            b.side = c->side;
+            b.fork = c->fork;
+            b.join = c->join;
+        }
         b.pairs = c->pairs.p;
         b.npairs = c->npairs.p;
         b.pcap = kPairCap;
@@ -1639,6 +1643,7 @@ int hdnnp_debug_fetch(hdnnp_ctx* c, const char* what, void* host, size_t bytes) 
     else if (w == "nei_rev") { src = b.nei_rev; n = sizeof(int) * b.nentries; }
     else if (w == "nsf_max") { tmp = c->model->dev.nsf_max; n = sizeof(int); }
     else if (w == "nentries") { tmp = b.nentries; n = sizeof(int); }
+    else if (w == "side_stream") { tmp = c->side != nullptr; n = sizeof(int); }
     else return fail(HDNNP_E_INPUT, "unknown item " + w);
     // list arrays: nentries is the reserved size (padded lists reserve more
     // than they fill); the leading entries the caller sized for are copied

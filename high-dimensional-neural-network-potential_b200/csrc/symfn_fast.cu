@@ -1403,8 +1403,11 @@ int nsm() { return device_sm_count(); }
 constexpr int kBlocksPerSm = 32;
 constexpr size_t kSmemSm = 228 * 1024;  // shared memory of an SM; 1 KB of every block is the system's
 
+//
+// query: only whether the pass would run as two launches (1 or 0).  Without a
+// list (b.wide null) it runs as one.
 template <typename T, class S, bool kB>
-int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
+int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query) {
     const int mfull = b.mmax > 0 ? ((b.mmax + 31) / 32) * 32 : 32;
     auto warp_bytes = [&](int mm) { return fast_warp_bytes<T, S>(mm, m.nel, m.g2max, m.nblk, grad); };
     // default split: the largest count at which the blocks the registers
@@ -1442,6 +1445,8 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
         warps_per_block(mfull, fit);
         if ((long long)b.natoms <= (long long)nsm() * fit) split = mfull;
     }
+    if (query) return mfull > split;
+    if (!b.wide) split = mfull;
     int L = 0;
     auto go = [&](int mm, int part, cudaStream_t on) {
         int fit;
@@ -1478,21 +1483,21 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
 
 // FP64: the form without exponential range tests where the potential allows it
 template <typename T, class S>
-int run_spec(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
+int run_spec(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query) {
     if constexpr (sizeof(T) == 8)
-        if (m.exp_bounded) return run_form<T, S, true>(b, m, grad, st);
-    return run_form<T, S, false>(b, m, grad, st);
+        if (m.exp_bounded) return run_form<T, S, true>(b, m, grad, st, query);
+    return run_form<T, S, false>(b, m, grad, st, query);
 }
 
 template <typename T>
-int run_any(const Batch& b, const DevModel& m, bool grad, cudaStream_t st) {
+int run_any(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query = false) {
     switch (m.fast) {
-        case 1: return run_spec<T, Spec<2, 2, 1>>(b, m, grad, st);
-        case 2: return run_spec<T, Spec<2, 4, 2>>(b, m, grad, st);
-        case 3: return run_spec<T, Spec<2, 4, 4>>(b, m, grad, st);
-        case 4: return run_spec<T, Spec<2, 8, 2>>(b, m, grad, st);
-        case 5: return run_spec<T, Spec<2, 2, 1, 1, 4>>(b, m, grad, st);
-        case 6: return run_spec<T, Spec<2, 4, 2, 1, 2, 4, 16>>(b, m, grad, st);
+        case 1: return run_spec<T, Spec<2, 2, 1>>(b, m, grad, st, query);
+        case 2: return run_spec<T, Spec<2, 4, 2>>(b, m, grad, st, query);
+        case 3: return run_spec<T, Spec<2, 4, 4>>(b, m, grad, st, query);
+        case 4: return run_spec<T, Spec<2, 8, 2>>(b, m, grad, st, query);
+        case 5: return run_spec<T, Spec<2, 2, 1, 1, 4>>(b, m, grad, st, query);
+        case 6: return run_spec<T, Spec<2, 4, 2, 1, 2, 4, 16>>(b, m, grad, st, query);
         default: return 0;
     }
 }
@@ -1508,6 +1513,11 @@ size_t sf_fast_smem_per_warp(int mmax, int g2max, int nblk, int P, bool grad, bo
     if (grad) n += 3 * a16(w * mm) + a16(sizeof(int) * mm) + a16(w * g2max) + 2 * a16(w * nblk * P);
     else n += a16(w * 32 * (P + 1)) + (fp32 ? a16(sizeof(double4) * mm) : 0);
     return n;
+}
+
+bool sf_fast_lists_atoms(const Batch& b, const DevModel& m, bool fp32) {
+    return fp32 ? run_any<float>(b, m, false, nullptr, true) || run_any<float>(b, m, true, nullptr, true)
+                : run_any<double>(b, m, false, nullptr, true) || run_any<double>(b, m, true, nullptr, true);
 }
 
 int launch_sf_values_fast(const Batch& b, const DevModel& m, bool fp32, cudaStream_t st) {

@@ -255,7 +255,8 @@ int hdnnp_dEdLat_to_stress(const double* lat, const double* dEdLat, double* stre
  * tests and profiling.  what: "G" (scaled symmetry functions, nat x nsf_max,
  * row stride nsf_max), "dEdG" (same layout), "atom_energy" (nat),
  * "nei_count" (nat, excluding the atom itself), "nei_index" (entries),
- * "nei_shift" (entries, packed image shift), "nsf_max" (1 int).
+ * "nei_shift" (entries, packed image shift), "nsf_max" (1 int),
+ * "side_stream" (1 int: whether the context has made its second stream).
  * `bytes` is the size of `host`; returns HDNNP_E_CAPACITY if too small.  The
  * list arrays ("nei_index", "nei_shift", "nei_rev") copy their first `bytes`
  * (size the buffer from "nei_count"): their reserved size can exceed the

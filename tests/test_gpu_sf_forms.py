@@ -224,3 +224,34 @@ def test_dense_batch_fills_the_gpu(pkg, W, tmp_path):
             assert best[0] <= 1.2 * best[-1], best
     finally:
         pot.close()
+
+
+@pytest.mark.parametrize("prec", ["FP64", "MIXED"])
+def test_second_stream_only_where_it_is_used(pkg, W, prec):
+    """A context makes its second stream when a batch first runs in two
+    launches: not for one cell (all its warps fit on the GPU), and not for a
+    batch when the option asks for one launch; the results are the same."""
+    from conftest import ABX3_DIR
+
+    from hdnnp_b200 import engine
+
+    pot = engine.Hdnnp.from_runner(ABX3_DIR)
+    try:
+        pot.set_precision(getattr(engine, "HDNNP_PREC_" + prec))
+        batch = W.config_c4(n_struct=96)
+
+        def made():
+            return int(pot.fetch("side_stream", 1, np.int32)[0])
+
+        pot.eval_batch(batch[:1])
+        assert made() == 0
+        pot.set_option("sf_split", -1)
+        one = pot.eval_batch(batch)
+        assert made() == 0
+        pot.set_option("sf_split", 0)
+        two = pot.eval_batch(batch)
+        assert made() == 1
+        for k in ("energy", "forces", "dEdLat"):
+            assert np.array_equal(one[k], two[k])
+    finally:
+        pot.close()
