@@ -212,7 +212,7 @@ def measured_peaks(torch):
 
 # Floating-point operations per work unit EXECUTED by the lambda x zeta x eta
 # symmetry-function kernels for the (2 lambda, zeta {1,2,4,16}, 2 eta) grid of
-# this potential, counted from csrc/symfn_fast.cu (add/mul = 1, FMA = 2,
+# this potential, counted from csrc/symfn_fast.cuh (add/mul = 1, FMA = 2,
 # sqrt/exp/tanh/div = 1).  Units come from the engine's counters.  The
 # product-space kernels execute about 9x fewer operations than the
 # reference's per-function loops; the roofline is therefore stated with the

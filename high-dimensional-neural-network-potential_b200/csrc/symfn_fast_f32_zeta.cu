@@ -1,0 +1,17 @@
+// symfn_fast_f32_zeta.cu -- FP32 kernels of the grid shapes whose zetas are read from
+// the model.
+#include "symfn_fast.cuh"
+
+namespace hdnnp {
+
+int run_sf_f32_zeta(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query) {
+    switch (m.fast) {
+        case 1: return run_spec<float, Spec<2, 2, 1>>(b, m, grad, st, query);
+        case 2: return run_spec<float, Spec<2, 4, 2>>(b, m, grad, st, query);
+        case 3: return run_spec<float, Spec<2, 4, 4>>(b, m, grad, st, query);
+        case 4: return run_spec<float, Spec<2, 8, 2>>(b, m, grad, st, query);
+        default: return 0;
+    }
+}
+
+}  // namespace hdnnp
