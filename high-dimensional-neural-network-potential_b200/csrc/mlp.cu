@@ -139,7 +139,7 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double bb) {
 }
 
 constexpr int kDW = 8;   // warps per block of k_mlp_split, one per atom of the tile
-constexpr int kRW = 10;  // warps per block of k_mlp_resident
+constexpr int kRW = 10;  // most warps per block of k_mlp_resident
 constexpr int kDH = 32;  // widest layer the kernels take
 constexpr int kDR = 8;   // atoms per tile
 // row stride of the activation rows: four rows of four doubles (the A
@@ -157,32 +157,29 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// The later layers' weights in shared memory, layer by layer the fragments of
-// the forward product ([ks][nt][32], B[k][n] = W[n][k]) and of the backward
-// product (B[k][n] = W[k][n]), zero-padded; doubles they take.
+// The later layers' weights in shared memory, layer by layer the fragments
+// [ks][nt][32] of the forward product (B[k][n] = W[n][k]), zero-padded to
+// whole tiles of 8 inputs; doubles they take.  The backward product reads the
+// same fragments transposed.
+__host__ __device__ inline int layer_doubles(const DevModel& m, int l) {
+    return 2 * ((m.width[l] + 7) >> 3) * ((m.width[l + 1] + 7) >> 3) * 32;
+}
 __host__ __device__ inline int hidden_doubles(const DevModel& m) {
     int h = 0;
-    for (int l = 1; l < m.nlayers; ++l) {
-        const int wi = m.width[l], wo = m.width[l + 1];
-        h += (((wi + 3) >> 2) * ((wo + 7) >> 3) + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
-    }
+    for (int l = 1; l < m.nlayers; ++l) h += layer_doubles(m, l);
     return h;
 }
 __device__ __forceinline__ void stage_hidden(const DevModel& m, int e, double* h, int tid, int nthreads) {
     const int L = m.nlayers;
     for (int l = 1; l < L; ++l) {
-        const int wi = m.width[l], wo = m.width[l + 1];
+        const int wi = m.width[l], wo = m.width[l + 1], NT = (wo + 7) >> 3, nf = layer_doubles(m, l);
         const double* W = m.w + m.w_off[e * L + l];  // [wo][wi]
-        for (int dir = 0; dir < 2; ++dir) {
-            const int kk = dir ? wo : wi, nn = dir ? wi : wo;
-            const int NT = (nn + 7) >> 3, nf = ((kk + 3) >> 2) * NT * 32;
-            for (int idx = tid; idx < nf; idx += nthreads) {
-                const int t = idx & 31, f = idx >> 5, n = (f % NT) * 8 + (t >> 2), k = 4 * (f / NT) + (t & 3);
-                if (n < nn && k < kk) cp_async8(h + idx, W + (dir ? (size_t)k * wi + n : (size_t)n * wi + k));
-                else h[idx] = 0.0;
-            }
-            h += nf;
+        for (int idx = tid; idx < nf; idx += nthreads) {
+            const int t = idx & 31, f = idx >> 5, n = (f % NT) * 8 + (t >> 2), k = 4 * (f / NT) + (t & 3);
+            if (n < wo && k < wi) cp_async8(h + idx, W + (size_t)n * wi + k);
+            else h[idx] = 0.0;
         }
+        h += nf;
     }
 }
 
@@ -201,6 +198,25 @@ __device__ __forceinline__ void rows_gemm(double (&acc)[NC][2], const double* ro
 #pragma unroll
         for (int nt = 0; nt < NC; ++nt)
             if (n0 + nt < NT) dmma(acc[nt], a, B[(ks * NT + n0 + nt) * 32 + lane]);
+    }
+}
+
+// The same with the transposed product B[k][n] = W[k][n]: element (k, n) lies
+// at thread 4 (k % 8) + n % 4 of the fragment [n / 4][k / 8], so a half-warp's
+// 16 elements are consecutive.  NTF: n-tiles of the stored (forward) product.
+template <int NC>
+__device__ __forceinline__ void rows_gemm_t(double (&acc)[NC][2], const double* rows, int k, const double* B, int NTF, int NT,
+                                            int n0, int r, int q, int lane) {
+#pragma unroll
+    for (int nt = 0; nt < NC; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+    const int KS = (k + 3) >> 2;
+    B += (lane >> 4) * NTF * 32 + (lane & 3) * 4 + ((lane >> 2) & 3);
+#pragma unroll 2
+    for (int ks = 0; ks < KS; ++ks) {
+        const double a = 4 * ks + q < k ? rows[r * kDS + 4 * ks + q] : 0.0;
+#pragma unroll
+        for (int nt = 0; nt < NC; ++nt)
+            if (n0 + nt < NT) dmma(acc[nt], a, B[(2 * (n0 + nt) * NTF + (ks >> 1)) * 32 + (ks & 1) * 16]);
     }
 }
 
@@ -298,7 +314,7 @@ __global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
         const int wi = m.width[l], wo = m.width[l + 1], NT = (wo + 7) >> 3;
         double acc[1][2];
         if (wib < NT) rows_gemm(acc, yrow, wi, h, NT, wib, r, q, lane);
-        h += (((wi + 3) >> 2) * NT + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
+        h += layer_doubles(m, l);
         __syncthreads();
         if (wib < NT)
 #pragma unroll
@@ -318,11 +334,10 @@ __global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
     const double* dl = da + (L - 1) * kDR * kDS;
     for (int l = L - 1; l >= 1; --l) {
         const int wi = m.width[l], wo = m.width[l + 1], NT = (wi + 7) >> 3;
-        const int nb = ((wo + 3) >> 2) * NT * 32;
         dl -= kDR * kDS;
         double acc[1][2];
-        if (wib < NT) rows_gemm(acc, yrow, wo, h - nb, NT, wib, r, q, lane);
-        h -= nb + ((wi + 3) >> 2) * ((wo + 7) >> 3) * 32;
+        h -= layer_doubles(m, l);
+        if (wib < NT) rows_gemm_t(acc, yrow, wo, h, (wo + 7) >> 3, NT, wib, r, q, lane);
         __syncthreads();
         if (wib < NT)
 #pragma unroll
@@ -362,13 +377,12 @@ __global__ void __launch_bounds__(32 * kDW) k_mlp_split(Batch b, DevModel m) {
 }
 
 // Shared memory of k_mlp_resident in doubles: W1 in the fragment orders of
-// layer 1 and of dE/dG, the later layers' weights in those of their forward
-// and backward products, biases, and per warp one activation/delta row set
-// and act'(c_l) of the layers but the last.
+// layer 1 and of dE/dG, the later layers' weights, biases, and for each of nw
+// warps one activation/delta row set and act'(c_l) of the layers but the last.
 struct DmmaLayout {
     int f1, b1, hid, bias, warps, total;
 };
-__host__ __device__ inline DmmaLayout dmma_layout(const DevModel& m, int nin) {
+__host__ __device__ inline DmmaLayout dmma_layout(const DevModel& m, int nin, int nw) {
     DmmaLayout o;
     const int H1 = m.width[1], L = m.nlayers;
     o.f1 = 0;
@@ -376,7 +390,7 @@ __host__ __device__ inline DmmaLayout dmma_layout(const DevModel& m, int nin) {
     o.hid = o.b1 + ((nin + 7) >> 3) * ((H1 + 3) >> 2) * 32;
     o.bias = o.hid + hidden_doubles(m);
     o.warps = o.bias + L * kDH;
-    o.total = o.warps + kRW * L * kDR * kDS;
+    o.total = o.warps + nw * L * kDR * kDS;
     return o;
 }
 
@@ -394,9 +408,9 @@ __host__ __device__ inline DmmaLayout dmma_layout(const DevModel& m, int nin) {
 template <bool kVec>
 __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel m, int nin_max) {
     extern __shared__ __align__(16) double dsm[];
-    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5, nw = blockDim.x >> 5;
     const int L = m.nlayers, H1 = m.width[1], nsf = m.nsf_max;
-    const DmmaLayout lo = dmma_layout(m, nin_max);
+    const DmmaLayout lo = dmma_layout(m, nin_max, nw);
     double* yrow = dsm + lo.warps + wib * L * kDR * kDS;
     double* da = yrow + kDR * kDS;
     const int r = lane >> 2, q = lane & 3;
@@ -419,17 +433,17 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
             // steps beyond the last one of an odd count are zero)
             const double* src = m.dm_fwd + m.dm_off_f[e];
             const int nf1 = ((nin + 3) >> 2) * 128;
-            for (int idx = tid; idx < KP * 256; idx += 32 * kRW) {
+            for (int idx = tid; idx < KP * 256; idx += 32 * nw) {
                 const int t = idx & 31, nt = (idx >> 5) & 3, ks = idx >> 7;
                 const int kk = 4 * (ks & 1) + (t & 3);
                 double* dst = dsm + lo.f1 + ((((ks & ~1) | (kk & 1)) * 4 + nt) << 5) + ((t & ~3) | (kk >> 1));
                 if (idx < nf1) cp_async8(dst, src + idx);
                 else *dst = 0.0;
             }
-            for (int idx = tid; idx < NB * KB * 32; idx += 32 * kRW)
+            for (int idx = tid; idx < NB * KB * 32; idx += 32 * nw)
                 cp_async8(dsm + lo.b1 + idx, m.dm_bwd + m.dm_off_b[e] + idx);
-            stage_hidden(m, e, dsm + lo.hid, tid, 32 * kRW);
-            for (int idx = tid; idx < L * kDH; idx += 32 * kRW) {
+            stage_hidden(m, e, dsm + lo.hid, tid, 32 * nw);
+            for (int idx = tid; idx < L * kDH; idx += 32 * nw) {
                 const int l = idx / kDH, n = idx % kDH;
                 dsm[lo.bias + idx] = n < m.width[l + 1] ? m.b[m.b_off[e * L + l] + n] : 0.0;
             }
@@ -464,9 +478,9 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
         int atom_n = atom_of(s0 + wib);
 #pragma unroll
         for (int i = 0; i < kCh; ++i) load(atom_n, i, an[i]);
-        for (int tile = s0 + wib; tile < s1; tile += kRW) {
+        for (int tile = s0 + wib; tile < s1; tile += nw) {
             const int atom = atom_n;
-            atom_n = atom_of(tile + kRW);
+            atom_n = atom_of(tile + nw);
             double acc[4][2], sum[4][2];  // a segment's products, the segments before it
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = sum[nt][0] = sum[nt][1] = 0.0;
@@ -506,7 +520,7 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
                 if (l > 0) {
                     const int wi = m.width[l];
                     rows_gemm(acc, yrow, wi, h, NT, 0, r, q, lane);
-                    h += (((wi + 3) >> 2) * NT + ((wo + 3) >> 2) * ((wi + 7) >> 3)) * 32;
+                    h += layer_doubles(m, l);
                     __syncwarp();
                 }
                 const char act = m.act[l];
@@ -532,9 +546,8 @@ __global__ void __launch_bounds__(32 * kRW, 1) k_mlp_resident(Batch b, DevModel 
             }
             for (int l = L - 1; l >= 1; --l) {
                 const int wi = m.width[l], wo = m.width[l + 1], NT = (wi + 7) >> 3;
-                const int nb = ((wo + 3) >> 2) * NT * 32;
-                rows_gemm(acc, yrow, wo, h - nb, NT, 0, r, q, lane);
-                h -= nb + ((wi + 3) >> 2) * ((wo + 7) >> 3) * 32;
+                h -= layer_doubles(m, l);
+                rows_gemm_t(acc, yrow, wo, h, (wo + 7) >> 3, NT, 0, r, q, lane);
                 __syncwarp();
 #pragma unroll
                 for (int nt = 0; nt < 4; ++nt)
@@ -617,11 +630,16 @@ void run_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
 
 // The tensor-core forms take networks whose layers are at most kDH wide,
 // with one output and at most 8 layers (dm_ok, set with the fragments at
-// model upload).  The resident form needs an element's weights to fit in
-// shared memory and enough tiles to keep its warps busy: its time for one
-// tile is long (53 us from 4,500 atoms down, against 18-35 us of the split
-// form).  Measured for 280-25-25-1 networks, split / resident: 93 / 88 us at
-// 18,000 atoms, 156 / 145 at 36,000.  Both give an atom the same bits.
+// model upload).  The resident form needs an element's weights and the rows of
+// at least kRWLeast warps in shared memory, and enough tiles to keep its warps
+// busy: its time for one tile is long (53 us from 4,500 atoms down, against
+// 18-35 us of the split form).  Measured for 280-25-25-1 networks, split /
+// resident: 93 / 88 us at 18,000 atoms, 156 / 145 at 36,000.  With fewer than
+// ten warps, 316,116 atoms, split / resident in ms: 280-25-25-25-1 (8 warps)
+// 1.24 / 0.98, 280-32-32-32-1 (7) 1.31 / 1.18, 280-25-25-25-25-1 (6) 1.79 /
+// 1.44; 280-30-30-30-30-1 (5) 1.85 / 1.79, but 0.286 / 0.296 at 40,272 atoms.
+// Both give an atom the same bits.
+constexpr int kRWLeast = 6;
 constexpr int kResidentTilesPerSm = 16;
 
 int launch_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
@@ -631,12 +649,16 @@ int launch_mlp(const Batch& b, const DevModel& m, cudaStream_t s) {
     }
     int nin = 0;
     for (int e = 0; e < m.nel; ++e) nin = nin > m.nin_el[e] ? nin : m.nin_el[e];
-    const size_t rsm = (size_t)dmma_layout(m, nin).total * sizeof(double);
+    // as many warps as fit beside the weights
+    int nw = kRW;
+    auto bytes = [&](int w) { return (size_t)dmma_layout(m, nin, w).total * sizeof(double); };
+    while (nw > kRWLeast && bytes(nw) > (size_t)kSmemLimit) --nw;
+    const size_t rsm = bytes(nw);
     const int nsm = device_sm_count();
     if (rsm <= (size_t)kSmemLimit && b.natoms >= nsm * kResidentTilesPerSm * kDR) {
         auto k = (m.nsf_max & 1) ? k_mlp_resident<false> : k_mlp_resident<true>;
         raise_smem_limit(k, rsm);
-        k<<<nsm, 32 * kRW, rsm, s>>>(b, m, nin);
+        k<<<nsm, 32 * nw, rsm, s>>>(b, m, nin);
         return 1;
     }
     const size_t smem = (size_t)split_doubles(m) * sizeof(double);
