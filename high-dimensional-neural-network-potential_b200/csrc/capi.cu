@@ -1305,7 +1305,7 @@ int hdnnp_ctx_set_option(hdnnp_ctx* c, const char* name, int value) {
         return HDNNP_OK;
     }
     if (std::string(name) == "nei_warp") {
-        if (value < -1 || value > 1) return fail(HDNNP_E_INPUT, "nei_warp must be -1, 0 or 1");
+        if (value < -1 || value > 2) return fail(HDNNP_E_INPUT, "nei_warp must be -1, 0, 1 or 2");
         c->nei_warp = value;
         return HDNNP_OK;
     }

@@ -872,8 +872,9 @@ int launch_neighbour_build_a(const Batch& b, const DevModel& m, cudaStream_t s, 
     }
     const unsigned gW = (unsigned)((32LL * b.natoms + kThreads - 1) / kThreads);
     if (b.pad_cap > 0) {  // plans: one search pass into padded rows
-        if (b.nei_warp == 0 && b.posc && b.natoms >= kCellListAtoms && b.natoms < kCellListMost &&
-            b.ncells <= kCellsPerAtom * (long long)b.natoms)
+        const bool cells = b.natoms >= kCellListAtoms && b.natoms < kCellListMost &&
+                           b.ncells <= kCellsPerAtom * (long long)b.natoms;
+        if (b.posc && (b.nei_warp == 2 || (b.nei_warp == 0 && cells)))
             k_neighbours_cell<<<(b.ncells + kCellWarps - 1) / kCellWarps, 32 * kCellWarps, 0, s>>>(b, m);
         else if (warp_lists(b))
             k_neighbours_warp<2><<<gW, kThreads, 0, s>>>(b, m);

@@ -107,8 +107,9 @@ int hdnnp_ctx_set_precision(hdnnp_ctx* c, int precision);
  * lambda x zeta x eta kernels read the zeta set from the model even when a
  * kernel with that zeta set compiled in exists.  Results agree within
  * rounding.  "nei_warp" chooses how neighbour lists are built: 1 one warp per
- * atom, -1 one thread per atom, 0 (default) a warp per atom below 131,072
- * atoms in the batch; both give the same lists, entry for entry.
+ * atom, -1 one thread per atom, 2 one warp per cell (one-pass lists: plans,
+ * and calls after a context's first; a warp per atom otherwise), 0 (default)
+ * by the batch's size; all give the same lists, entry for entry.
  * "small_eval" (default 1): a call of one molecule of at most 64 atoms in
  * FP64 (the reference's own MD example is one) runs as one kernel launch, a
  * thread block that builds the lists by direct search and keeps every
