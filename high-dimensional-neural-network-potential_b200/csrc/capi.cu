@@ -863,11 +863,8 @@ int run_pipeline(hdnnp_ctx* c, int nstruct, int natoms, const int32_t* Zd, const
         b.virf = c->virf.p;
     }
     {
-        int mm = ((b.mmax + 31) / 32) * 32;
-        const size_t sf_smem =
-            fast ? sf_fast_smem_per_warp(mm, D.g2max, D.nblk, fast_shape_p(D.fast), true, mixed) * 4
-                   : sf_smem_per_warp(mm, true) * 4;
-        if (sf_smem > 220 * 1024 || (fast && mm > 1024))
+        const int mm = ((b.mmax + 31) / 32) * 32;
+        if (fast ? !sf_fast_takes(b, D, mixed) : sf_smem_per_warp(mm, true) * 4 > 220 * 1024)
             return fail(HDNNP_E_CAPACITY, "too many neighbours per atom for the symmetry-function kernels");
         if (mlp_smem_bytes(D, mixed ? sizeof(float) : sizeof(double)) > 220 * 1024)
             return fail(HDNNP_E_CAPACITY, "network too wide for the MLP kernel");

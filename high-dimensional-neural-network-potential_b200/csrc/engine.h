@@ -388,11 +388,15 @@ constexpr int kFastZeta[kNumFastShapes][4] = {{0}, {0}, {0}, {0}, {0}, {1, 4, 0,
 inline int fast_shape_p(int id) { return kFastShapes[id][0] * kFastShapes[id][1] * kFastShapes[id][2]; }
 
 // Fast (product-space) symmetry-function kernels, FP64 (T = double) or FP32.
+// what the product-space passes are asked without a launch: whether one lists
+// atoms for a second launch, whether its layout takes the largest count
+enum class SfAsk { kNothing, kLists, kFits };
+// whether the passes take the batch's largest neighbour count
+bool sf_fast_takes(const Batch& b, const DevModel& m, bool fp32);
 // whether a pass over the batch lists atoms for a second launch (Batch::wide,
 // side, fork and join are then needed)
 bool sf_fast_lists_atoms(const Batch& b, const DevModel& m, bool fp32);
 int launch_sf_values_fast(const Batch& b, const DevModel& m, bool fp32, cudaStream_t s);
 int launch_sf_gradients_fast(const Batch& b, const DevModel& m, bool fp32, cudaStream_t s);
-size_t sf_fast_smem_per_warp(int mmax, int g2max, int nblk, int P, bool grad, bool fp32);
 
 }  // namespace hdnnp

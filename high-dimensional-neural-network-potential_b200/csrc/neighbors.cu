@@ -171,10 +171,6 @@ __device__ __forceinline__ int cand(const Batch& b, int p, double& x, double& y,
     return j;
 }
 
-// floor(a / n) for n > 0, in integers (the same value as the floating-point
-// floor of the exact quotient)
-__device__ __forceinline__ int floor_div(int a, int n) { return a >= 0 ? a / n : -((n - 1 - a) / n); }
-
 // Wrap a cell coordinate c into [0, n) and return the image count floor(c / n):
 // the search offsets reach at most nsearch cells beyond the grid, so this is
 // one step for grids of at least nsearch cells and a few for tiny cells --

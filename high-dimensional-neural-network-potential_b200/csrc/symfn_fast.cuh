@@ -254,7 +254,6 @@ __device__ __forceinline__ void dist_inv(float r2, float& r, float& ir) {
 // b between 2^-126 and 2^126)
 __device__ __forceinline__ double xdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ float xdiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double xexp(double x) { return exp_clamped(x); }
 // FP32 form: the exp2-based intrinsic (max error 2 + floor(1.173 |x|) ulp;
 // the angular arguments stay below ~5, where it is within 8 ulp)
 __device__ __forceinline__ float xexp(float x) { return __expf(x); }
@@ -563,17 +562,7 @@ __device__ __forceinline__ T pair_u(const FSmem<T>& s, int j, int k, double rc2d
 }
 
 // ---------------------------------------------------------------- powers
-// X^E from the square chain ch[b] = X^(2^b); E is a compile-time constant
-// after unrolling, so the bit tests fold away.
-template <int E, typename T>
-__device__ __forceinline__ T cpow(const T (&ch)[5]) {
-    T r = (T)1;
-#pragma unroll
-    for (int bit = 0; bit < 5; ++bit)
-        if ((E >> bit) & 1) r = r * ch[bit];
-    return r;
-}
-
+// X^e from the square chain ch[b] = X^(2^b)
 template <typename T>
 __device__ __forceinline__ T rpow(const T (&ch)[5], int e) {
     T r = (T)1;
@@ -1212,10 +1201,10 @@ __device__ __forceinline__ void grad_pairs(const FSmem<T>& s, const DevModel& m,
         }
 }
 
-template <typename T, class S, bool kB>
 // Bound by instruction issue and shared-memory latency: per pair two dozen
 // 16-byte shared loads, the geometry, cutoff, exponentials and powers again,
 // the contraction with dE/dG, and the update of two slots.
+template <typename T, class S, bool kB>
 __global__ void __launch_bounds__(32 * kWarps, kBlocksG<T>) k_sfg_fast(Batch b, DevModel m, int mm, int part) {
     constexpr int NL = S::NL, NZ = S::NZ, NE = S::NE, P = S::P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1410,12 +1399,14 @@ constexpr int kBlocksPerSm = 32;
 constexpr size_t kSmemSm = 228 * 1024;  // shared memory of an SM; 1 KB of every block is the system's
 
 //
-// query: only whether the pass would run as two launches (1 or 0).  Without a
-// list (b.wide null) it runs as one.
+// ask: only an answer (1 or 0), no launch.  Without a list (b.wide null) the
+// pass runs as one launch.
 template <typename T, class S, bool kB>
-int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query) {
+int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, SfAsk ask) {
     const int mfull = b.mmax > 0 ? ((b.mmax + 31) / 32) * 32 : 32;
     auto warp_bytes = [&](int mm) { return fast_warp_bytes<T, S>(mm, m.nel, m.g2max, m.nblk, grad); };
+    // (slots are 10 bits in the pair lists)
+    if (ask == SfAsk::kFits) return mfull <= 1024 && warp_bytes(mfull) <= (size_t)kSmemLimit;
     // default split: the largest count at which the blocks the registers
     // allow still fit (1 KB of every block is the system's)
     const int resident = grad ? kBlocksG<T> : kBlocksV<T>;
@@ -1451,7 +1442,7 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool
         warps_per_block(mfull, fit);
         if ((long long)b.natoms <= (long long)nsm() * fit) split = mfull;
     }
-    if (query) return mfull > split;
+    if (ask == SfAsk::kLists) return mfull > split;
     if (!b.wide) split = mfull;
     int L = 0;
     auto go = [&](int mm, int part, cudaStream_t on) {
@@ -1489,10 +1480,10 @@ int run_form(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool
 
 // FP64: the form without exponential range tests where the potential allows it
 template <typename T, class S>
-int run_spec(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query) {
+int run_spec(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, SfAsk ask) {
     if constexpr (sizeof(T) == 8)
-        if (m.exp_bounded) return run_form<T, S, true>(b, m, grad, st, query);
-    return run_form<T, S, false>(b, m, grad, st, query);
+        if (m.exp_bounded) return run_form<T, S, true>(b, m, grad, st, ask);
+    return run_form<T, S, false>(b, m, grad, st, ask);
 }
 
 }  // namespace

@@ -3,10 +3,10 @@
 
 namespace hdnnp {
 
-int run_sf_f32(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query) {
+int run_sf_f32(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, SfAsk ask) {
     switch (m.fast) {
-        case 5: return run_spec<float, Spec<2, 2, 1, 1, 4>>(b, m, grad, st, query);
-        case 6: return run_spec<float, Spec<2, 4, 2, 1, 2, 4, 16>>(b, m, grad, st, query);
+        case 5: return run_spec<float, Spec<2, 2, 1, 1, 4>>(b, m, grad, st, ask);
+        case 6: return run_spec<float, Spec<2, 4, 2, 1, 2, 4, 16>>(b, m, grad, st, ask);
         default: return 0;
     }
 }

@@ -4,12 +4,12 @@
 
 namespace hdnnp {
 
-int run_sf_f32_zeta(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, bool query) {
+int run_sf_f32_zeta(const Batch& b, const DevModel& m, bool grad, cudaStream_t st, SfAsk ask) {
     switch (m.fast) {
-        case 1: return run_spec<float, Spec<2, 2, 1>>(b, m, grad, st, query);
-        case 2: return run_spec<float, Spec<2, 4, 2>>(b, m, grad, st, query);
-        case 3: return run_spec<float, Spec<2, 4, 4>>(b, m, grad, st, query);
-        case 4: return run_spec<float, Spec<2, 8, 2>>(b, m, grad, st, query);
+        case 1: return run_spec<float, Spec<2, 2, 1>>(b, m, grad, st, ask);
+        case 2: return run_spec<float, Spec<2, 4, 2>>(b, m, grad, st, ask);
+        case 3: return run_spec<float, Spec<2, 4, 4>>(b, m, grad, st, ask);
+        case 4: return run_spec<float, Spec<2, 8, 2>>(b, m, grad, st, ask);
         default: return 0;
     }
 }
