@@ -831,8 +831,10 @@ constexpr int kCellsPerAtom = 4;
 // thread per atom from 131,072 atoms) / a warp per cell, in us: 42 / 59 at 768
 // atoms, 125 / 116 at 18,000, 355 / 290 at 71,000, 723 / 637 at 191,000.
 constexpr int kCellListAtoms = 12288;
-// Largest one: from here a thread per atom keeps the GPU full (1.93 ms of the
-// 758,676-atom step, against about 2.6).
+// Largest one: from here a thread per atom keeps the 148 SMs full.  List
+// stages with a thread per atom / a warp per cell, in us: 796 / 705 at 187,284
+// atoms, 905 / 925 at 262,488, 992 / 1,091 at 316,116, 1,461 / 1,654 at
+// 500,088, 1,979 / 2,441 at 758,676; one cell of 294,912 atoms 794 / 916.
 constexpr int kCellListMost = 262144;
 
 // Batches whose list stages run in one block each: up to kSmallAtoms atoms the

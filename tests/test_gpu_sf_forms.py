@@ -2,9 +2,11 @@
 accepts, against the FP64 oracle: grids of one, two and four etas and up to
 eight zetas (accumulator tiles, several passes over the partner elements),
 exponents inside and beyond the range of the form without range tests, centre
-elements without functions for some element pairs; centres without pairs,
-with more neighbours than the first launch takes and with more pairs than the
-pair list holds.
+elements without functions for some element pairs; centres without pairs and
+with more pairs than the pair list holds (the oracle's batch is small enough
+for one launch; test_gpu_edges.py compares the two launches of a pass with
+one, bit for bit).  Scaling, collinear atoms, the dense batch's launches, the
+second stream.
 
 FP64: |dE| <= 1e-10 |E|, max |dF|, |d dE/dh| <= 1e-9 times the largest force
 (at least 1).  Mixed precision: 1e-4 of the largest force, the FP32 rounding
